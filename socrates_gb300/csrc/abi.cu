@@ -512,7 +512,30 @@ int build_spectrum(const socgpu_spectrum_desc *d, SpectrumEntry &e, char *msg, s
   };
   std::vector<float> grid_f(grid.begin(), grid.end()), k_lk_f(k_lk.begin(), k_lk.end());
   std::vector<float> tgas_f(tgas.begin(), tgas.end()), wy_f(wy.begin(), wy.end());
-  if (!up(s.bands_keqv, bands_keqv) || !up(s.gpoints_keqv, gpoints_keqv) || !up(s.minor_terms, minor) ||
+  std::vector<BandLite> lite(s.n_band);
+  for (int b = 0; b < s.n_band; ++b) {
+    const BandInfo &bi = e.bands_host[b];
+    const BandGas &g = bi.gas[0];
+    BandLite &t = lite[b];
+    t = BandLite{};
+    t.n_abs = bi.n_abs; t.n_cont = bi.n_cont; t.rayleigh = bi.rayleigh_f; t.solar = bi.solar_flux_band_f;
+    t.species = g.species; t.i_scale_k = g.i_scale_k; t.i_scale_fnc = g.i_scale_fnc; t.l_doppler = g.l_doppler;
+    t.p_ref = g.p_ref_f; t.t_ref = g.t_ref_f; t.doppler_cor = g.doppler_cor_f;
+    std::copy(g.scale_f, g.scale_f + 4, t.scale);
+    // sum_k c_k x^k about x = 1: the synthetic divisions of Horner's scheme
+    double c[kMaxPlanckCoeff];
+    std::copy(bi.planck, bi.planck + kMaxPlanckCoeff, c);
+    for (int j = 0; j < kMaxPlanckCoeff; ++j)
+      for (int k = kMaxPlanckCoeff - 2; k >= j; --k) c[k] += c[k + 1];
+    std::copy(c, c + kMaxPlanckCoeff, t.planck);
+    if (b > 0) {
+      const BandLite &u = lite[b - 1];
+      t.same = t.i_scale_fnc == u.i_scale_fnc && t.l_doppler == u.l_doppler && t.p_ref == u.p_ref &&
+               t.t_ref == u.t_ref && t.doppler_cor == u.doppler_cor && t.i_scale_k == u.i_scale_k &&
+               std::equal(t.scale, t.scale + 4, u.scale);
+    }
+  }
+  if (!up(s.lite, lite) || !up(s.bands_keqv, bands_keqv) || !up(s.gpoints_keqv, gpoints_keqv) || !up(s.minor_terms, minor) ||
       !up(s.lk_grid, grid) || !up(s.lk_grid_f, grid_f) || !up(s.k_lookup, k_lk) || !up(s.k_lookup_f, k_lk_f) ||
       !up(s.t_lookup_gas, tgas) || !up(s.t_lookup_gas_f, tgas_f) || !up(s.wenyi, wy) || !up(s.wenyi_f, wy_f) ||
       !up(s.aer_tab, aer_tab) || !up(s.aer_tab_f, aer_tab_f) || !up(s.aer_hum, aer_hum) ||
@@ -563,6 +586,7 @@ void free_spectrum(SpectrumEntry &e) {
   cudaFree(e.dev.aer_hum);
   cudaFree(e.dev.aer_hum_f);
   cudaFree(e.dev.bands);
+  cudaFree(e.dev.lite);
   cudaFree(e.dev.gpoints);
   cudaFree(e.dev.drop_parm);
   cudaFree(e.dev.ice_parm);
@@ -623,18 +647,39 @@ std::mutex g_tile_mutex;
 int g_tile[2][3][2] = {};   // [precision][mode][lanes, warps]
 std::map<std::tuple<int, int, int>, TileConfig> g_tuned;
 
-// The built-in scan tile: 32 lanes above 64 layers (mixed) or above 128
-// layers (FP64), else 16; 8 warps; the smallest chunk covering the column.
-TileConfig scan_tile(int precision, int n_layer) {
+// Lanes per solve of the built-in tile.  FP64: 16 up to 128 layers, else 32.
+// Mixed clear skies: 8 up to 104 layers, 16 up to 144, else 32 -- few lanes
+// mean few scan steps per layer, as long as a lane's layers fit in 128
+// registers (measured on GB300, us: solar 10000 x 100 455 with 8 lanes, 485
+// with 16, 627 with 32; scattering long wave 3001 x 137 377 with 16, 443 with
+// 32, 575 with 8).  McICA and equivalent extinction: 16 up to 64 layers, else
+// 32 (solar McICA 8000 x 85 1252 with 32, 1453 with 8; GA9 short wave 2000 x
+// 70 329 with 32, 342 with 16, 430 with 8): the lanes of a McICA warp then
+// share a subcolumn, and the minor absorbers' solves spread over more lanes.
+int built_in_lanes(int precision, int mode, int n_layer, bool keqv) {
+  if (precision != SOCGPU_PRECISION_MIXED) return n_layer <= 128 ? 16 : 32;
+  if (mode == 2 || keqv) return n_layer <= 64 ? 16 : 32;
+  return n_layer <= 104 ? 8 : n_layer <= 144 ? 16 : 32;
+}
+
+// Warps per CTA of the built-in tile: under equivalent extinction, whose
+// minor absorbers leave lanes idle, four (GA9 short wave 2000 x 70 329 us, 350
+// with 8) unless the columns are too few to fill the SMs.
+int built_in_warps(int precision, bool keqv, int nd_profile) {
+  return precision == SOCGPU_PRECISION_MIXED && keqv && nd_profile > 304 ? 4 : 8;
+}
+
+// The built-in scan tile, with the smallest chunk covering the column.
+TileConfig scan_tile(int precision, int mode, int n_layer, bool keqv, int nd_profile) {
   TileConfig t{};
-  t.lanes_per_solve = precision == SOCGPU_PRECISION_MIXED ? (n_layer <= 64 ? 16 : 32) : (n_layer <= 128 ? 16 : 32);
-  t.warps_per_cta = 8;
+  t.lanes_per_solve = built_in_lanes(precision, mode, n_layer, keqv);
+  t.warps_per_cta = built_in_warps(precision, keqv, nd_profile);
   while (t.lanes_per_solve < 32 && smallest_chunk(precision, t.lanes_per_solve, n_layer) == 0) t.lanes_per_solve *= 2;
   t.chunk = smallest_chunk(precision, t.lanes_per_solve, n_layer);
   return t;
 }
 
-TileConfig choose_tile(int precision, int mode, int n_layer) {
+TileConfig choose_tile(int precision, int mode, int n_layer, bool keqv, int nd_profile) {
   TileConfig t{};
   bool tuned = false;
   {
@@ -647,13 +692,8 @@ TileConfig choose_tile(int precision, int mode, int n_layer) {
     }
   }
   if (!tuned) {
-    if (t.lanes_per_solve <= 0) {
-      // measured on GB300: short chunks (few layers per lane) win over long
-      // ones -- fewer live registers and more resident warps
-      if (precision == SOCGPU_PRECISION_MIXED) t.lanes_per_solve = n_layer <= 64 ? 16 : 32;
-      else t.lanes_per_solve = n_layer <= 128 ? 16 : 32;
-    }
-    if (t.warps_per_cta <= 0) t.warps_per_cta = 8;
+    if (t.lanes_per_solve <= 0) t.lanes_per_solve = built_in_lanes(precision, mode, n_layer, keqv);
+    if (t.warps_per_cta <= 0) t.warps_per_cta = built_in_warps(precision, keqv, nd_profile);
     t.chunk = 0;
   }
   // the phased kernel's chunk is its k-term batch (0: the launcher's default)
@@ -970,6 +1010,7 @@ void fill_params(FluxParams &p, const socgpu_control *c, const socgpu_dimen *dm,
   for (int b = c->first_band - 1; b < c->last_band; ++b)
     p.max_abs = std::max(p.max_abs, c->l_gas ? sp->bands_host[b].n_abs : 0);
   p.bands = p.keqv ? sp->dev.bands_keqv : sp->dev.bands;
+  p.lite = sp->dev.lite;
   p.gpoints = p.keqv ? sp->dev.gpoints_keqv : sp->dev.gpoints;
   p.minor_terms = sp->dev.minor_terms;
   // lookup tables (staged per column only when a band of the range uses them)
@@ -1110,9 +1151,9 @@ int launch(const FluxParams &p, const socgpu_control *c, cudaStream_t st, char *
 namespace {
 int launch_flux(const FluxParams &p, const socgpu_control *c, cudaStream_t st, char *msg, size_t msg_len) {
   const int mode = mode_index(c);
-  TileConfig t = choose_tile(c->precision, mode, p.n_layer);
+  TileConfig t = choose_tile(c->precision, mode, p.n_layer, p.keqv, p.nd_profile);
   // options the phased kernel does not cover run on the scan kernels
-  if (t.lanes_per_solve == 1 && !phased_supported(p)) t = scan_tile(c->precision, p.n_layer);
+  if (t.lanes_per_solve == 1 && !phased_supported(p)) t = scan_tile(c->precision, mode, p.n_layer, p.keqv, p.nd_profile);
   const FluxVariant *v = find_variant(c->precision, mode, t.lanes_per_solve);
   if (v && t.lanes_per_solve == 1) return v->launch(p, t, st, msg, msg_len);
   if (!v || t.chunk == 0) {
@@ -1577,13 +1618,13 @@ int launch_group(const BatchGroup &g, FluxParams *di, long long *ds, cudaStream_
 // Group the batches by the tile each one is given (tuner table, overrides or
 // heuristic), prepare, upload and capture the graph.
 int build_plan(socgpu_batch_s &b, char *msg, size_t msg_len) {
-  std::map<std::tuple<int, int, int, int, int, int>, std::vector<int>> classes;
+  std::map<std::tuple<int, int, int, int, int, int, int>, std::vector<int>> classes;
   for (size_t i = 0; i < b.params.size(); ++i) {
-    TileConfig t = choose_tile(b.precision[i], b.mode[i], b.params[i].n_layer);
+    TileConfig t = choose_tile(b.precision[i], b.mode[i], b.params[i].n_layer, b.params[i].keqv, b.params[i].nd_profile);
     // the phased kernel has no persistent multi-batch form
-    if (t.lanes_per_solve == 1) t = scan_tile(b.precision[i], b.params[i].n_layer);
+    if (t.lanes_per_solve == 1) t = scan_tile(b.precision[i], b.mode[i], b.params[i].n_layer, b.params[i].keqv, b.params[i].nd_profile);
     classes[std::make_tuple(b.precision[i], b.mode[i], t.lanes_per_solve, t.chunk, t.warps_per_cta,
-                            b.params[i].isolir)].push_back((int)i);
+                            b.params[i].isolir, b.params[i].region)].push_back((int)i);
   }
   b.groups.assign(classes.size(), BatchGroup{});
   b.group_items.assign(classes.size(), {});
@@ -1982,13 +2023,14 @@ int socgpu_batch_tune(socgpu_batch batch, void *stream, int reps, char *msg, siz
       if (!find_variant(prec, mode, lanes) || chunk == 0) continue;
       for (int warps : {4, 8}) {
         TileConfig t{lanes, warps, chunk};
-        // one group per source
-        std::vector<std::vector<int>> by_src(2);
-        for (int i : kv.second) by_src[b.params[i].isolir == SOCGPU_IP_SOLAR ? 0 : 1].push_back(i);
+        // one group per source, cloud regions apart
+        std::vector<std::vector<int>> by_src(4);
+        for (int i : kv.second)
+          by_src[(b.params[i].isolir == SOCGPU_IP_SOLAR ? 0 : 1) + (b.params[i].region ? 2 : 0)].push_back(i);
         std::vector<BatchGroup> groups;
         std::vector<std::vector<FluxParams>> items;
         std::vector<std::vector<long long>> starts;
-        groups.reserve(2); items.reserve(2); starts.reserve(2);
+        groups.reserve(4); items.reserve(4); starts.reserve(4);
         bool fits = true;
         for (auto &idx : by_src) {
           if (idx.empty()) continue;

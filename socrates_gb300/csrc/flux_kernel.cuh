@@ -53,19 +53,19 @@ __device__ __forceinline__ double ld2(const double *a, int l, int i, int nd) {
 // (the F2F instruction issues on the FP64 pipe).  Results below the FP32
 // normal range flush to zero, as the mixed kernels run with FTZ; NaN stays
 // NaN and overflow gives infinity.
+static __device__ __noinline__ unsigned narrow_large(unsigned mag, unsigned lo) {   // overflow, infinity, NaN
+  return (mag > 0x7FF00000u || (mag == 0x7FF00000u && lo)) ? 0x7FC00000u : 0x7F800000u;
+}
 __device__ __forceinline__ float narrow(double d) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
-  const unsigned sign = hi & 0x80000000u;
-  const int e = (int)((hi >> 20) & 0x7FFu) - 1023 + 127;
-  const unsigned m = ((hi & 0xFFFFFu) << 3) | (lo >> 29);
-  const unsigned rem = lo & 0x1FFFFFFFu;
-  unsigned bits = ((unsigned)e << 23) + m;
-  bits += (rem > 0x10000000u) | ((rem == 0x10000000u) & (m & 1u));
-  if (e <= 0) bits = 0u;
-  if (e >= 255) bits = ((hi & 0x7FFFFFFFu) > 0x7FF00000u || ((hi & 0x7FFFFFFFu) == 0x7FF00000u && lo))
-                           ? 0x7FC00000u : 0x7F800000u;
-  return __uint_as_float(sign | bits);
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  // the low nine exponent bits and 23 fraction bits, rebiased by 1023 - 127
+  // (its low nine bits are 384); the rounding carry may step the exponent
+  const unsigned x = __funnelshift_l(lo, hi, 3);
+  const unsigned up = ((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (x & 1u)) >> 29;
+  const unsigned mag = hi & 0x7FFFFFFFu;
+  unsigned bits = mag < 0x38100000u ? 0u : x + up - 0xC0000000u;
+  if (mag >= 0x47F00000u) bits = narrow_large(mag, lo);
+  return __uint_as_float((hi & 0x80000000u) | bits);
 }
 
 // FP32 -> FP64 widening (exact) on the integer pipe; FP32 subnormals are
@@ -433,12 +433,16 @@ struct FluxKernel {
   struct Smem {
     R *p, *t, *mass, *kgt, *kes, *kabs, *asym, *fwd, *amt, *bscal, *planck, *dB, *dB2;
     R *phf_nc, *fwd_nc, *c_ke, *c_ks, *c_ka, *c_phf, *c_fwd, *wcld, *frac, *csub;
-    R *aux, *lkf, *sbf, *kscr;
+    R *aux, *lkf, *sbf, *scr;    // scr: this thread's group's scratch row
     int *lki, *sbj;
     R *ovl, *reg, *t0d, *frr;
     double *regd;
     int *nct;
     Acc *acc;
+    // the mixed kernels' depths and accumulators (flux_tau_kernel.cuh)
+    float4 *opt, *copt;
+    float *tkd, *pl, *accd;
+    float2 *acc2;
     // the column's raw inputs (null: read them from global memory)
     const double *raw;
     int r_p, r_t, r_mass, r_gas, r_mmr, r_mabs, r_msca, r_masy, r_sol, r_zen, r_alb, r_tg, r_fg, r_tl;
@@ -458,7 +462,7 @@ struct FluxKernel {
     s.aux = (R *)(smem + l.off_aux);
     s.lkf = (R *)(smem + l.off_lkf); s.lki = (int *)(smem + l.off_lki);
     s.sbf = (R *)(smem + l.off_sbf); s.sbj = (int *)(smem + l.off_sbj);
-    s.kscr = (R *)(smem + l.off_kscr);
+    s.scr = (R *)(smem + l.off_kscr) + (size_t)(threadIdx.x / P) * LP;
     s.ovl = (R *)(smem + l.off_ovl); s.reg = (R *)(smem + l.off_reg); s.nct = (int *)(smem + l.off_nct);
     s.regd = (double *)(smem + l.off_regd);
     s.t0d = (R *)(smem + l.off_t0d);
@@ -1095,6 +1099,26 @@ struct FluxKernel {
   // (opt_prop_water_cloud.F90:231-247, opt_prop_ice_cloud.F90:278-294) and
   // Fu's ice fits (opt_prop_fu_phf_mod.F90:92-130).  Forward scattering is
   // k_scat g^2 (n_order_forward 2) for all of them.
+  __device__ static __forceinline__ void cloud_optics(int scheme, bool ice, const R *cp, R re, R qm, R &kext, R &coalb,
+                                                      R &g) {
+    if (scheme == SOCGPU_IP_SLINGO_SCHRECKER) {
+      // the droplet and ice forms are the same (both schemes are 1)
+      kext = qm * (cp[0] + cp[1] / re);
+      coalb = cp[2] + cp[3] * re;
+      g = cp[4] + cp[5] * re;
+    } else if (scheme == SOCGPU_IP_ICE_FU_PHF && ice) {
+      R x = cp[3] / re;
+      kext = qm * ((cp[2] * x + cp[1]) * x + cp[0]);
+      x = re / cp[8];
+      coalb = cp[4] + x * (cp[5] + x * (cp[6] + x * cp[7]));
+      x = re / cp[13];
+      g = cp[9] + x * (cp[10] + x * (cp[11] + x * cp[12]));
+    } else {
+      kext = qm * (cp[0] + re * (cp[1] + re * cp[2])) / (R(1) + re * (cp[3] + re * (cp[4] + re * cp[5])));
+      coalb = (cp[6] + re * (cp[7] + re * cp[8])) / (R(1) + re * (cp[9] + re * cp[10]));
+      g = (cp[11] + re * (cp[12] + re * cp[13])) / (R(1) + re * (cp[14] + re * cp[15]));
+    }
+  }
   __device__ static void stage_cloud_bands(const FluxParams &p, const Smem &S, int col, int bstart, int nb) {
     const int L = p.n_layer, ndp = p.nd_profile, ndl = p.nd_layer, ict = p.id_ct;
     const int ndc = ndl - ict, nc = p.n_condensed;
@@ -1116,25 +1140,8 @@ struct FluxKernel {
             const float *c = (p.comp_phase[k] == SOCGPU_IP_PHASE_WATER ? p.drop_parm_f : p.ice_parm_f) + po;
             for (int m = 0; m < kCloudParm; ++m) cp[m] = c[m];
           }
-          const int scheme = p.comp_scheme[k];
           R kext, coalb, g;
-          if (scheme == SOCGPU_IP_SLINGO_SCHRECKER) {
-            // the droplet and ice forms are the same (both schemes are 1)
-            kext = qm * (cp[0] + cp[1] / re);
-            coalb = cp[2] + cp[3] * re;
-            g = cp[4] + cp[5] * re;
-          } else if (scheme == SOCGPU_IP_ICE_FU_PHF && p.comp_phase[k] == SOCGPU_IP_PHASE_ICE) {
-            R x = cp[3] / re;
-            kext = qm * ((cp[2] * x + cp[1]) * x + cp[0]);
-            x = re / cp[8];
-            coalb = cp[4] + x * (cp[5] + x * (cp[6] + x * cp[7]));
-            x = re / cp[13];
-            g = cp[9] + x * (cp[10] + x * (cp[11] + x * cp[12]));
-          } else {
-            kext = qm * (cp[0] + re * (cp[1] + re * cp[2])) / (R(1) + re * (cp[3] + re * (cp[4] + re * cp[5])));
-            coalb = (cp[6] + re * (cp[7] + re * cp[8])) / (R(1) + re * (cp[9] + re * cp[10]));
-            g = (cp[11] + re * (cp[12] + re * cp[13])) / (R(1) + re * (cp[14] + re * cp[15]));
-          }
+          cloud_optics(p.comp_scheme[k], p.comp_phase[k] == SOCGPU_IP_PHASE_ICE, cp, re, qm, kext, coalb, g);
           const R kscat = kext * (R(1) - coalb);
           vke = kext; vks = kscat; vka = kext * coalb; vph = kscat * g; vfw = kscat * g * g;
         }
@@ -1238,7 +1245,7 @@ struct FluxKernel {
                                                     const GPoint &gp, const BandInfo &bd, const R *amt, int r, int L,
                                                     R (&kgv)[CH]) {
     if (p.l_gas && gt.any_term) {
-      R *scr = S.kscr + (size_t)(threadIdx.x / P) * LP;
+      R *scr = S.scr;
       gas_k_terms(p, S, gp, bd, gt.n_abs, amt, r, L, scr);
 #pragma unroll
       for (int jj = 0; jj < CH; ++jj) kgv[jj] = scr[jj * P + r];
@@ -1256,7 +1263,7 @@ struct FluxKernel {
   __device__ static __forceinline__ void term_k_lane(const FluxParams &p, const Smem &S, const BandGas &gs, int b,
                                                      R kj, const R *sc, int lk_off, int iex, const R *amt, int r,
                                                      int L, R (&kk)[CH]) {
-    R *scr = S.kscr + (size_t)(threadIdx.x / P) * LP;
+    R *scr = S.scr;
     const Lk lk = lk_of(S);
 #pragma unroll 1
     for (int jj = 0; jj < CH; ++jj) {
@@ -1532,7 +1539,11 @@ struct FluxKernel {
     // the unscaled direct transmissions (i_direct_tau = ip_direct_noscaling)
     R *t0d = (!lw && p.i_direct_tau == SOCGPU_IP_DIRECT_NOSCALING && !p.region)
                  ? S.t0d + (size_t)(threadIdx.x / P) * LP : nullptr;
-    if (!MCICA) {
+    if constexpr (!kFP64 && P > 1) {
+      // the mixed kernels solve clear skies and McICA in optical-depth form
+      // (flux_tau_kernel.cuh); cloud regions come here
+      solve_region(p, g, bstart, sec0, r, lw, active);
+    } else if constexpr (!MCICA) {
       // the gas absorption of the lane's layers first, while few registers
       // are live, then the coefficients
       R kgv[CH];
@@ -2369,7 +2380,8 @@ struct FluxKernel {
   }
 
   // Sources, direct beam, solve and accumulation of one monochromatic
-  // problem held in the group's registers.
+  // problem held in the group's registers (FP64; the mixed kernels' solve is
+  // in flux_tau.cuh).
   __device__ static void solve_column(const FluxParams &p, R (&T)[CH], R (&Rf)[CH], R (&T0)[CH],
                                       R (&c1)[CH], R (&c2)[CH], R (&om)[CH], int r, int L, bool lw,
                                       const R *dB_b, const R *dB2_b, R f_inc_down, R f_inc_dir,
@@ -2379,10 +2391,6 @@ struct FluxKernel {
     const int L_acc = active ? L : -1;
     Acc *acc_up = acc, *acc_dn = acc + (LP + 1), *acc_dir = acc + 2 * (LP + 1), *acc_div = acc + 3 * (LP + 1);
     // --- sources -------------------------------------------------------------
-    // ssum = s_up + s_down of each layer: with om = 1 - T - R it gives the
-    // layer's flux divergence (1-T-R)(F_dn(top) + F_up(bottom)) - ssum, the
-    // form the mixed kernel uses instead of differencing FP32 level fluxes
-    R ssum[CH];
     R fdir_bottom = R(0);
     if (!lw) {
       // direct beam: exclusive product scan of the chunks' transmissions
@@ -2408,7 +2416,6 @@ struct FluxKernel {
         const int i = r * CH + j;
         R su = c1[j] * fd, sd = c2[j] * fd;   // solar_source.F90:146-155
         c1[j] = su; c2[j] = sd;
-        ssum[j] = su + sd;
         fd = fd * T0[j];
         if (i < L_dir) acc_dir[j * P + r] += w * fd;
       }
@@ -2446,14 +2453,12 @@ struct FluxKernel {
           if (p.l_ir_source_quad) {       // ir_source.F90:93-119
             su = c1[j] * dB + c2[j] * dB2_b[s];
             sd = -c1[j] * dB + c2[j] * dB2_b[s];
-            ssum[j] = R(2) * c2[j] * dB2_b[s];
           } else {
             su = c1[j] * dB; sd = -su;
-            ssum[j] = R(0);
           }
           c1[j] = su; c2[j] = sd;
         } else {
-          c1[j] = R(0); c2[j] = R(0); ssum[j] = R(0);
+          c1[j] = R(0); c2[j] = R(0);
         }
       }
     }
@@ -2506,8 +2511,7 @@ struct FluxKernel {
         if (i < L_acc) {
           acc_up[s] += w * c1[j];
           acc_dn[s] += w * fdn;
-          if constexpr (kFP64) acc_div[s] += w * (c1[j] - fu_prev + fd - fdn);
-          else acc_div[s] += w * (om[j] * (fd + c1[j]) - ssum[j]);
+          acc_div[s] += w * (c1[j] - fu_prev + fd - fdn);
         }
         fu_prev = c1[j];
         fd = fdn;
@@ -2588,8 +2592,7 @@ struct FluxKernel {
       if (i < L_acc) {
         acc_up[s] += w * fu;
         acc_dn[s] += w * fd;
-        if constexpr (kFP64) acc_div[s] += w * (fu - fu_top + fd_top - fd);
-        else acc_div[s] += w * (om[j] * (fd_top + fu) - ssum[j]);
+        acc_div[s] += w * (fu - fu_top + fd_top - fd);
       }
       fu = fu_top; fd = fd_top;
     }

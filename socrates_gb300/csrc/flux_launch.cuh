@@ -5,11 +5,112 @@
 #include <algorithm>
 #include <cstdio>
 #include "flux_kernel.cuh"
+#include "flux_tau_kernel.cuh"
 
 namespace socgpu {
 
 template <int P_, int CH_>
 struct Shape { static constexpr int P = P_, CH = CH_; };
+
+// Whether batch p runs on the mixed kernels in optical-depth form.
+template <class R, bool MCICA>
+constexpr bool tau_form(const FluxParams &p) { return sizeof(R) == 4 && !(MCICA && p.region); }
+
+// Shared memory the current device grants one CTA.
+inline int smem_limit() {
+  int v = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return v;
+}
+
+// One batch on the mixed kernel of shape S.
+template <bool NOSCAT, bool MCICA, int SRC, class S>
+int launch_tau(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char *msg, size_t len) {
+  FluxParams q = p;
+  int warps = cfg.warps_per_cta;
+  const size_t cap = (size_t)smem_limit();
+  while (!tau_fit(q, S::P * S::CH, S::P, warps, MCICA, cap)) {
+    if (warps == 1) {
+      snprintf(msg, len, "one band of %d layers needs %u bytes of shared memory (limit %zu)", p.n_layer, q.tau.stride, cap);
+      return SOCGPU_I_ERR_RANGE;
+    }
+    warps /= 2;
+  }
+  const size_t bytes = tau_bytes(q);
+  auto kern = tau_kernel<S::P, S::CH, NOSCAT, MCICA, SRC>;
+  if (bytes > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
+      return SOCGPU_I_ERR_RANGE;
+    }
+  }
+  if (p.n_profile <= 0) return 0;
+  kern<<<(p.n_profile + q.tau.cols - 1) / q.tau.cols, warps * 32, bytes, st>>>(q);
+  count_launch();
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    snprintf(msg, len, "flux kernel launch failed: %s", cudaGetErrorString(e));
+    return SOCGPU_I_ABORT_CALCULATION;
+  }
+  return 0;
+}
+
+// One kernel class on the mixed kernel of shape S: every item's layout, the
+// work in column groups, and a persistent grid.
+template <bool NOSCAT, bool MCICA, int SRC, class S>
+int prepare_tau(BatchGroup &g, char *msg, size_t len) {
+  int dev = 0, n_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  const int warps = g.tile.warps_per_cta;
+  auto kern = tau_kernel_batched<S::P, S::CH, NOSCAT, MCICA, SRC>;
+  cudaFuncAttributes fa{};
+  if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) {
+    cudaGetLastError();
+    snprintf(msg, len, "attributes of the batched kernel not available");
+    return SOCGPU_I_ABORT_CALCULATION;
+  }
+  // the kernel's static shared memory (its parameter copy) counts too
+  const size_t cap = (size_t)smem_limit() - std::min((size_t)smem_limit(), fa.sharedSizeBytes);
+  size_t bytes = 0;
+  for (int i = 0; i < g.n_items; ++i) {
+    FluxParams &p = g.items[i];
+    if (p.n_layer > S::P * S::CH) {
+      snprintf(msg, len, "batch %d has %d layers, more than the %d of its tile", i, p.n_layer, S::P * S::CH);
+      return SOCGPU_I_ERR_RANGE;
+    }
+    if (!tau_fit(p, S::P * S::CH, S::P, warps, MCICA, cap)) {
+      snprintf(msg, len, "batch %d: one band needs %u bytes of shared memory (limit %zu)", i, p.tau.stride, cap);
+      return SOCGPU_I_ERR_RANGE;
+    }
+    bytes = std::max(bytes, tau_bytes(p));
+    g.col_start[i + 1] = g.col_start[i] + (p.n_profile + p.tau.cols - 1) / p.tau.cols;
+  }
+  g.total = g.col_start[g.n_items];
+  if (bytes > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
+      return SOCGPU_I_ERR_RANGE;
+    }
+  }
+  int per_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, bytes);
+  if (e != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    snprintf(msg, len, "no CTA of %d threads and %zu bytes fits an SM", warps * 32, bytes);
+    return SOCGPU_I_ERR_RANGE;
+  }
+  g.kernel = (const void *)kern;
+  g.smem = bytes;
+  g.threads = warps * 32;
+  g.grid = (int)std::min<long long>(g.total, (long long)per_sm * n_sm);
+  return 0;
+}
 
 template <class R, bool MIX, bool NOSCAT, bool MCICA, int SRC, class S>
 int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char *msg, size_t len,
@@ -19,6 +120,10 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   // the smallest chunk of this P that covers the column is chosen by the
   // caller's ordering of shapes (ascending CH)
   done = true;
+  if constexpr (sizeof(R) == 4) {
+    if (tau_form<R, MCICA>(p)) return launch_tau<NOSCAT, MCICA, SRC, S>(p, cfg, st, msg, len);
+  }
+  if constexpr (sizeof(R) == 8 || MCICA) {
   const int nb = p.last_band - p.first_band + 1;
   int max_smem = 0, dev = 0;
   cudaGetDevice(&dev);
@@ -56,6 +161,7 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
     snprintf(msg, len, "flux kernel launch failed: %s", cudaGetErrorString(e));
     return SOCGPU_I_ABORT_CALCULATION;
   }
+  }
   return 0;
 }
 
@@ -66,6 +172,11 @@ template <class R, bool MIX, bool NOSCAT, bool MCICA, int SRC, class S>
 int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
   if (done || g.tile.lanes_per_solve != S::P || g.tile.chunk != S::CH) return 0;
   done = true;
+  if constexpr (sizeof(R) == 4) {
+    // a class holds cloud regions only, or none (its key says which)
+    if (g.n_items == 0 || tau_form<R, MCICA>(g.items[0])) return prepare_tau<NOSCAT, MCICA, SRC, S>(g, msg, len);
+  }
+  if constexpr (sizeof(R) == 8 || MCICA) {
   int max_smem = 0, dev = 0, n_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -129,6 +240,7 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
   g.smem = dyn;
   g.threads = warps * 32;
   g.grid = (int)std::min<long long>(g.total, (long long)per_sm * n_sm);
+  }
   return 0;
 }
 
@@ -184,9 +296,15 @@ template <class R, bool MIX, bool NOSCAT, bool MCICA, int SRC, int P, int... CH>
 int preload_chunks() {
   cudaFuncAttributes a{};
   bool ok = true;
-  ((ok = ok && cudaFuncGetAttributes(&a, flux_kernel<R, MIX, P, CH, NOSCAT, MCICA, SRC>) == cudaSuccess), ...);
-  ((ok = ok && cudaFuncGetAttributes(&a, flux_kernel_batched<R, MIX, P, CH, NOSCAT, MCICA, SRC>) == cudaSuccess),
-   ...);
+  if constexpr (sizeof(R) == 8 || MCICA) {
+    ((ok = ok && cudaFuncGetAttributes(&a, flux_kernel<R, MIX, P, CH, NOSCAT, MCICA, SRC>) == cudaSuccess), ...);
+    ((ok = ok && cudaFuncGetAttributes(&a, flux_kernel_batched<R, MIX, P, CH, NOSCAT, MCICA, SRC>) == cudaSuccess),
+     ...);
+  }
+  if constexpr (sizeof(R) == 4) {
+    ((ok = ok && cudaFuncGetAttributes(&a, tau_kernel<P, CH, NOSCAT, MCICA, SRC>) == cudaSuccess), ...);
+    ((ok = ok && cudaFuncGetAttributes(&a, tau_kernel_batched<P, CH, NOSCAT, MCICA, SRC>) == cudaSuccess), ...);
+  }
   if (!ok) cudaGetLastError();
   return ok ? 0 : SOCGPU_I_ABORT_CALCULATION;
 }

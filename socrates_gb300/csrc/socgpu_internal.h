@@ -66,6 +66,20 @@ struct BandInfo {
   int minor_first[kMaxAbsPerBand], minor_count[kMaxAbsPerBand];
 };
 
+// What the staging of the mixed kernels reads of a band, for every layer: a
+// 128-byte record, copied to shared memory (a BandInfo is some 2 KB).
+struct BandLite {
+  int n_abs, n_cont;
+  float rayleigh, solar;            // Rayleigh coefficient, fraction of the solar constant
+  // the first absorber
+  int species, i_scale_k, i_scale_fnc, l_doppler;
+  float p_ref, t_ref, doppler_cor, scale[4];
+  int same;                         // scaled as the first absorber of the band before
+  float planck[kMaxPlanckCoeff];    // Planck polynomial in T / T_ref - 1
+  int pad[4];
+};
+static_assert(sizeof(BandLite) == 128, "copied as 32 words");
+
 // One k-term of one absorber of a band: the minor gases of k_eqv_scl.
 struct TermK {
   int iex;                          // 0-based k-term
@@ -100,6 +114,7 @@ struct SpectrumDev {
   int has_solar, has_planck, has_rayleigh, has_continuum, index_water;
   int n_drop_type, n_ice_type;
   BandInfo *bands;                  // [n_band]
+  BandLite *lite;                   // [n_band]
   GPoint *gpoints;                  // [n_gpoint]
   int random_ok;                    // the random-overlap products fit SOCGPU_MAX_GPOINT
   // equivalent extinction: the major absorber's terms as g-points, the minor
@@ -139,6 +154,19 @@ struct SpectrumDev {
   int host_first_g[SOCGPU_MAX_BAND + 1];
 };
 
+// Shared memory of a CTA of the mixed kernels (flux_tau_kernel.cuh), filled
+// by the host: cols columns of `stride` bytes each, and in each column the
+// offsets (bytes) of its arrays for nbat bands staged at a time.
+struct TauLayout {
+  int cols;                         // adjacent columns of a CTA (1, 2 or 4)
+  int warps;                        // warps that share a column's g-points
+  int nbat;                         // bands staged at a time
+  int acc_stride, accd_stride;      // accumulators of a group: (up, divergence) pairs, direct fluxes
+  unsigned stride;
+  unsigned opt, copt, tkd, amt, aux, bscal, planck, dB, dB2, pl, p, t, mass, frac, csub, lkf, lki, sbf, sbj, scr;
+  unsigned acc2, accd;
+};
+
 // Everything a flux kernel launch reads, as device pointers with the
 // caller's Fortran leading extents.
 struct FluxParams {
@@ -158,6 +186,7 @@ struct FluxParams {
   int band_batch;                   // bands staged in shared memory at a time (set by the launcher)
   // spectrum
   const BandInfo *bands;
+  const BandLite *lite;
   const GPoint *gpoints;
   const double *drop_parm, *ice_parm;
   const float *drop_parm_f, *ice_parm_f;
@@ -235,6 +264,7 @@ struct FluxParams {
   double dp_corr[3];                 // decorrelation scales [Pa] of the clear, stratiform, convective regions
   int triple;                        // three regions: clear, stratiform and convective (ip_cloud_triple)
   int type_region[4];                // the region (2 stratiform, 3 convective) of each 0-based cloud type
+  TauLayout tau;                     // the mixed kernels' shared memory (set by the launcher)
 };
 
 // Launch configuration chosen by the tuner.
@@ -253,7 +283,8 @@ struct BatchGroup {
   long long *col_start = nullptr;     // host array [n_items + 1]
   int n_items = 0;
   long long total = 0;                // columns of all batches
-  // filled by the prepare step
+  // filled by the prepare step (the mixed kernels' col_start and total
+  // become counts of CTAs' column groups there)
   const void *kernel = nullptr;
   size_t smem = 0;
   int threads = 0, grid = 0;
@@ -262,7 +293,7 @@ struct BatchGroup {
 // Layers per lane (CH) instantiated for each precision and lane count P; a
 // kernel covers P * CH layers.  flux_inst.cu is compiled once per
 // (precision, mode, P) and instantiates these chunks.
-#define SOCGPU_CHUNKS_MIXED_8  5, 8, 13, 18
+#define SOCGPU_CHUNKS_MIXED_8  5, 8, 9, 11, 13, 18
 #define SOCGPU_CHUNKS_MIXED_16 3, 4, 5, 7, 9, 16
 #define SOCGPU_CHUNKS_MIXED_32 3, 4, 5, 8, 16
 #define SOCGPU_CHUNKS_FP64_16  4, 8, 16
