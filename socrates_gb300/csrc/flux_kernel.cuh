@@ -1240,11 +1240,30 @@ struct FluxKernel {
     }
   }
 
+  // One absorber whose k comes from a (pressure, temperature) table: the
+  // mixed kernels read the tables of all the lane's layers together (a rolled
+  // loop waits for the four gathers of each layer in turn).
+  __device__ static __forceinline__ bool lookup_only(const BandGas &gs, int n_abs) {
+    return !kFP64 && n_abs == 1 && gs.i_scale_k == SOCGPU_IP_SCALE_TERM &&
+           gs.i_scale_fnc == SOCGPU_IP_SCALE_LOOKUP && gs.sb < 0;
+  }
+  __device__ static __forceinline__ void lookup_lane(const FluxParams &p, const Smem &S, int off, const R *amt, int r,
+                                                     int L, R (&kk)[CH]) {
+    const Lk lk = lk_of(S);
+#pragma unroll
+    for (int jj = 0; jj < CH; ++jj) {
+      const int i = r * CH + jj, s = jj * P + r;
+      kk[jj] = i < L ? lookup_k(p, lk, off, -1, s, amt[s]) : R(0);
+    }
+  }
+
   // The gas absorption of a g-point in the lane's layers.
   __device__ static __forceinline__ void gas_k_lane(const FluxParams &p, const Smem &S, const GasTerm &gt,
                                                     const GPoint &gp, const BandInfo &bd, const R *amt, int r, int L,
                                                     R (&kgv)[CH]) {
-    if (p.l_gas && gt.any_term) {
+    if (lookup_only(bd.gas[0], gt.n_abs) && p.l_gas) {
+      lookup_lane(p, S, gp.lk_off[0], amt, r, L, kgv);
+    } else if (p.l_gas && gt.any_term) {
       R *scr = S.scr;
       gas_k_terms(p, S, gp, bd, gt.n_abs, amt, r, L, scr);
 #pragma unroll
@@ -1263,6 +1282,10 @@ struct FluxKernel {
   __device__ static __forceinline__ void term_k_lane(const FluxParams &p, const Smem &S, const BandGas &gs, int b,
                                                      R kj, const R *sc, int lk_off, int iex, const R *amt, int r,
                                                      int L, R (&kk)[CH]) {
+    if (lookup_only(gs, 1)) {
+      lookup_lane(p, S, lk_off, amt, r, L, kk);
+      return;
+    }
     R *scr = S.scr;
     const Lk lk = lk_of(S);
 #pragma unroll 1
@@ -1336,7 +1359,7 @@ struct FluxKernel {
           const int i = r * CH + jj, s = jj * P + r;
           if (i < L) {
             if constexpr (kFP64) e[jj] = exp(-kk[jj] * S.mass[s] * sec0);
-            else e[jj] = expf(-kk[jj] * S.mass[s] * sec0);
+            else e[jj] = __expf(-kk[jj] * S.mass[s] * sec0);
           } else {
             e[jj] = R(1);
           }
@@ -1356,7 +1379,7 @@ struct FluxKernel {
         for (int jj = 0; jj < CH; ++jj) {
           if constexpr (!kFP64) {
             const int s = jj * P + r;
-            if (r * CH + jj < L) loss[s] += f * -expm1f(-kk[jj] * S.mass[s] * sec0);
+            if (r * CH + jj < L) loss[s] += f * one_minus_exp(kk[jj] * S.mass[s] * sec0, e[jj]);
           }
           f = f * e[jj];
           fg[jj] += f;

@@ -81,9 +81,11 @@ inline size_t tau_bytes(const FluxParams &p) {
 // one.  Measured on GB300 (us, mixed, 8 warps): solar 10000 x 100 454 with
 // four columns, 475 with two, 715 with one; long wave 1000 x 60 39, 52, 78;
 // scattering long wave 3001 x 137 377 (bands in batches), 364, 393; solar
-// McICA 8000 x 85 1400 (in batches), 1252, 1445.  Equivalent extinction keeps
-// four and stages its bands in batches: the minor absorbers dominate (GA9
-// short wave 2000 x 70 329 us, 354 with two).
+// McICA 8000 x 85 1400 (in batches), 1252, 1445.  Under equivalent
+// extinction the minor absorbers dominate: a CTA of 4 warps takes 87, 150
+// and 270 us for one, two and four columns of the GA9 short wave, however few
+// share its SM, so the count with the least waves times that is taken (2000 x
+// 70: 327, 305, 280 us; 2500 x 70: 402, 444, 531).
 // The rule looks at the leading extent, not at the number of columns of the
 // call, so that a window of a batch sums in the same order as the whole.
 // False: one band of one column does not fit.
@@ -92,7 +94,12 @@ inline bool tau_fit(FluxParams &p, int LP, int P, int warps_cta, bool mcica, siz
   const int nb_all = p.last_band - p.first_band + 1;
   const size_t want = std::min(cap, (size_t)(227 * 1024) * warps_cta / 16);
   const int resident = kTauResident * 8 / warps_cta;
-  const int most = warps_cta % 4 != 0 || p.nd_profile <= resident ? 1 : p.nd_profile <= 2 * resident ? 2 : 4;
+  int most = warps_cta % 4 != 0 || p.nd_profile <= resident ? 1 : p.nd_profile <= 2 * resident ? 2 : 4;
+  if (p.keqv && most == 4) {
+    const auto waves = [&](int c) { return (double)((p.nd_profile + c * resident - 1) / (c * resident)); };
+    const double t1 = waves(1), t2 = 1.72 * waves(2), t4 = 3.1 * waves(4);
+    most = t4 <= t1 && t4 <= t2 ? 4 : t2 <= t1 ? 2 : 1;
+  }
   for (int cols = most; cols >= 1; cols /= 2) {
     const int least = cols == 4 ? (p.keqv ? 1 : nb_all) : cols == 2 ? (nb_all + 1) / 2 : 1;
     for (int nb = nb_all; nb >= least; --nb) {
