@@ -56,20 +56,145 @@ struct GenArgs {
 };
 
 // First and last layer holding cloud in any column (socrates_cloud_gen.F90:225-250).
+// One atomic per warp that improves the range: an atomic per cloudy cell
+// serialised on the two words.
 __global__ void cloud_range_kernel(GenArgs a) {
-  const int ndc = a.nd_layer - a.cloud_top + 1;
   const int ncol = a.il2 - a.il1 + 1;
   const long long total = (long long)ncol * (a.n_layer - a.cloud_top + 1);
   const double cut = kEps64;
+  int lo = a.n_layer + 1, hi = a.cloud_top - 1;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
        q += (long long)gridDim.x * blockDim.x) {
-    int il = a.il1 + (int)(q % ncol);
-    int k = a.cloud_top + (int)(q / ncol);
-    double cf = a.avg_cf[(size_t)(il - 1) + (size_t)a.nd_profile * (size_t)(k - a.cloud_top)];
-    if (cf > cut) atomicMin(&a.range[0], k);
-    if (cf >= cut) atomicMax(&a.range[1], k);
+    const int kk = (int)(q / ncol), il = a.il1 + (int)(q - (long long)kk * ncol), k = a.cloud_top + kk;
+    const double cf = a.avg_cf[(size_t)(il - 1) + (size_t)a.nd_profile * (size_t)kk];
+    if (cf > cut) lo = min(lo, k);
+    if (cf >= cut) hi = max(hi, k);
   }
-  (void)ndc;
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) {
+    if (lo <= a.n_layer) atomicMin(&a.range[0], lo);
+    if (hi >= a.cloud_top) atomicMax(&a.range[1], hi);
+  }
+}
+
+#define CLD(arr, k) __ldg((arr) + (size_t)(il - 1) + (size_t)ndp * (size_t)((k) - ct))
+#define CSUB(k, s) a.c_sub[(size_t)(il - 1) + (size_t)ndp * ((size_t)((k) - ct) + (size_t)ndc * (size_t)((s) - 1))]
+
+// The decorrelation of layer k with the one above (socrates_cloud_gen.F90:
+// 338-380): exp of the pressure (height) step over the decorrelation scale.
+__device__ __forceinline__ double cloud_alpha(const GenArgs &a, const double *scale, int il, int km) {
+  const int ndp = a.nd_profile, ct = a.cloud_top;
+  const double dz = __dsub_rn(__ldg(a.zf + (size_t)(il - 1) + (size_t)ndp * (size_t)(km - 1)),
+                              __ldg(a.zf + (size_t)(il - 1) + (size_t)ndp * (size_t)km));
+  const double l = CLD(scale, km);
+  return l > 0.0 ? exp(__ddiv_rn(dz, l)) : 0.0;
+}
+
+// Philox, no condensate variance (ipph = 0), random or exponential-random
+// overlap: the generator spread over subcolumns.
+//
+// With one thread per column the 16 subcolumns of a column follow one another
+// (8192 x 85 x 16: 823 us, 8192 threads on 152 SMs, each a serial chain of
+// FP64 arithmetic).  Here a CTA owns 32 columns, lane = column, and its warps
+// take the subcolumns.  What a layer's draws are compared with is the same in
+// all of them, so it is formed once per (layer, column): the deviates are
+// w 2^-32 with w an integer, hence x1 >= alpha is w1 >= ceil(alpha 2^32) and
+// x < cf is w < ceil(cf 2^32) -- exact, and integer arithmetic in the loop (the
+// FP64 pipe runs at 1/64 of FP32).  Without condensate variance the second
+// deviate (y) decides nothing.  The masks are kept as bits until the number of
+// cloudy subcolumns before each is known; then every element of c_sub is
+// written once, 32 columns together.  Same masks bit for bit; 8192 x 85 x 16 now
+// takes 56 us, of which its stores (89 MB) need 13.
+//
+// A subcolumn starts from the deviate the one before it ended with.  That
+// matters only if the first cloudy layer is correlated with the layer above
+// it (a cloud fraction at or below epsilon there); such a column's warps walk
+// through the earlier subcolumns first.
+struct GenShared {
+  unsigned long long *reset, *cloudy;     // [layers][32] thresholds; cloudy 0: no cloud
+  unsigned *bits;                         // [n_subcol][words][32]
+};
+__host__ __device__ inline size_t gen_shared_bytes(int ncl, int n_subcol) {
+  return (size_t)ncl * 32 * 16 + (size_t)n_subcol * ((ncl + 31) / 32) * 32 * 4;
+}
+
+__device__ __forceinline__ unsigned long long ceil_2_32(double v) {     // min(ceil(v 2^32), 2^32); v > 0
+  const double c = ceil(v * 4294967296.0);
+  return c < 4294967296.0 ? (unsigned long long)c : 4294967296ull;
+}
+
+__global__ void __launch_bounds__(512) cloud_gen_philox_kernel(GenArgs a, int ncl) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int ndp = a.nd_profile, ct = a.cloud_top, ndc = a.nd_layer - ct + 1;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, words = (ncl + 31) / 32;
+  GenShared sh;
+  sh.reset = (unsigned long long *)smem;
+  sh.cloudy = sh.reset + (size_t)ncl * 32;
+  sh.bits = (unsigned *)(sh.cloudy + (size_t)ncl * 32);
+  const int il_own = a.il1 + blockIdx.x * 32 + lane;
+  const bool own = il_own <= a.il2;
+  const int il = own ? il_own : a.il2;
+  const int k_top = a.range[0], k_base = a.range[1];
+  const int nk = (k_top > a.n_layer || k_base < k_top) ? 0 : k_base - k_top + 1;   // <= ncl
+  for (int q = w; q < nk; q += nw) {
+    const int k = k_top + q, km = k - 1;
+    const double cf = CLD(a.avg_cf, k);
+    unsigned long long f = 0, r = 0;
+    if (cf > 0.0) {
+      f = ceil_2_32(cf);
+      if (a.ioverlap != SOCGPU_IP_RAND && km >= ct && CLD(a.avg_cf, km) > 0.0) {
+        const double alpha = cloud_alpha(a, a.rlc_cf, il, km);
+        // a NaN is never reached, zero always
+        r = alpha > 0.0 ? ceil_2_32(alpha) : alpha == 0.0 ? 0ull : 4294967296ull;
+      }
+    }
+    sh.reset[q * 32 + lane] = r;
+    sh.cloudy[q * 32 + lane] = f;
+  }
+  __syncthreads();
+  int q1 = 0;
+  while (q1 < nk && sh.cloudy[q1 * 32 + lane] == 0) ++q1;
+  const bool carry = q1 < nk && sh.reset[q1 * 32 + lane] != 0;
+  const uint32_t key0 = (uint32_t)a.rand_seed[il - 1], key1 = 0x534F4352u;
+  for (int i = 1 + w; i <= a.n_subcol; i += nw) {
+    unsigned *bits = sh.bits + (size_t)(i - 1) * words * 32 + lane;
+    uint32_t x = 0;
+    for (int ii = carry ? 1 : i; ii <= i; ++ii) {
+      unsigned word = 0;
+      for (int q = 0; q < nk; ++q) {
+        const unsigned long long f = sh.cloudy[q * 32 + lane];
+        if (f != 0) {
+          uint32_t u[4];
+          philox4x32_10((uint32_t)(k_top + q), (uint32_t)ii, 0u, 0u, key0, key1, u);
+          if (u[0] >= sh.reset[q * 32 + lane]) x = u[2];
+          if (x < f) word |= 1u << (q & 31);
+        }
+        if ((q & 31) == 31 || q == nk - 1) { bits[(q >> 5) * 32] = word; word = 0; }
+      }
+    }
+  }
+  __syncthreads();
+  // output slot t takes the t-th subcolumn that holds cloud; the rest are clear
+  for (int t = w; t < a.n_subcol; t += nw) {
+    int src = -1, n_cld = 0;
+    for (int i = 0; i < a.n_subcol && nk > 0; ++i) {
+      unsigned any = 0;
+      for (int v = 0; v < (nk + 31) / 32; ++v) any |= sh.bits[((size_t)i * words + v) * 32 + lane];
+      if (any) {
+        if (n_cld == t) src = i;
+        ++n_cld;
+      }
+    }
+    if (!own) continue;
+    if (t == 0) a.n_subcol_cld[il - 1] = n_cld;
+    const unsigned *bits = sh.bits + (size_t)(src < 0 ? 0 : src) * words * 32 + lane;
+    for (int k = ct; k <= a.nd_layer; ++k) {
+      const int q = k - k_top;
+      const bool on = src >= 0 && q >= 0 && q < nk && (bits[(q >> 5) * 32] >> (q & 31) & 1u);
+      CSUB(k, t + 1) = on ? 1.0 : 0.0;
+    }
+  }
 }
 
 __global__ void cloud_gen_kernel(GenArgs a) {
@@ -77,8 +202,6 @@ __global__ void cloud_gen_kernel(GenArgs a) {
   if (il > a.il2) return;
   const int ndp = a.nd_profile, ct = a.cloud_top, ndc = a.nd_layer - ct + 1;
   const double rm = 1.0 / (double)kM;
-#define CLD(arr, k) __ldg((arr) + (size_t)(il - 1) + (size_t)ndp * (size_t)((k) - ct))
-#define CSUB(k, s) a.c_sub[(size_t)(il - 1) + (size_t)ndp * ((size_t)((k) - ct) + (size_t)ndc * (size_t)((s) - 1))]
   for (int s = 1; s <= a.n_subcol; ++s)
     for (int k = ct; k <= a.nd_layer; ++k) CSUB(k, s) = 0.0;
   const int k_top = a.range[0], k_base = a.range[1];
@@ -140,11 +263,8 @@ __global__ void cloud_gen_kernel(GenArgs a) {
         const int km = k - 1;
         if (!(a.ioverlap == SOCGPU_IP_RAND || km < ct)) {
           if (a.ioverlap == SOCGPU_IP_EXPONENTIAL || CLD(a.avg_cf, km) > 0.0) {
-            double dz = __dsub_rn(__ldg(a.zf + (size_t)(il - 1) + (size_t)ndp * (size_t)(km - 1)),
-                                  __ldg(a.zf + (size_t)(il - 1) + (size_t)ndp * (size_t)km));
-            double lcf = CLD(a.rlc_cf, km), lcw = CLD(a.rlc_cw, km);
-            alpha = lcf > 0.0 ? exp(__ddiv_rn(dz, lcf)) : 0.0;
-            rcorr = lcw > 0.0 ? exp(__ddiv_rn(dz, lcw)) : 0.0;
+            alpha = cloud_alpha(a, a.rlc_cf, il, km);
+            rcorr = cloud_alpha(a, a.rlc_cw, il, km);
           }
         }
         double x1, y1;
@@ -216,6 +336,25 @@ static int gen_block(int ncol) {
   return std::min(128, std::max(32, (per + 31) / 32 * 32));
 }
 
+// The generator over a batch whose cloudy layer range is known on the device:
+// the Philox kernel where it applies and its tables fit in shared memory, the
+// one-thread-per-column kernel otherwise.
+static cudaError_t launch_generator(const GenArgs &a, cudaStream_t st) {
+  const int ncol = a.il2 - a.il1 + 1, ncl = a.n_layer - a.cloud_top + 1;
+  const size_t bytes = gen_shared_bytes(std::max(ncl, 1), a.n_subcol);
+  if (a.rng == SOCGPU_RNG_PHILOX && a.ipph == 0 &&
+      (a.ioverlap == SOCGPU_IP_RAND || a.ioverlap == SOCGPU_IP_EXPONENTIAL_RAND) && bytes <= 100 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(cloud_gen_philox_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    cloud_gen_philox_kernel<<<(ncol + 31) / 32, 32 * std::min(16, a.n_subcol), bytes, st>>>(a, std::max(ncl, 1));
+  } else {
+    const int bs = gen_block(ncol);
+    cloud_gen_kernel<<<(ncol + bs - 1) / bs, bs, 0, st>>>(a);
+  }
+  count_launch();
+  return cudaGetLastError();
+}
+
 int launch_cloud_gen(int nd_layer, int cloud_top, int n_layer, int nd_profile, int il1, int il2,
                      int n_subcol, int n1, int n2, int ipph, int ioverlap, const int *rand_seed,
                      const double *rlc_cf, const double *rlc_cw, const double *sigma_qcw,
@@ -231,14 +370,11 @@ int launch_cloud_gen(int nd_layer, int cloud_top, int n_layer, int nd_profile, i
   cudaMemcpyAsync(range_dev, init, sizeof(init), cudaMemcpyHostToDevice, st);
   long long cells = (long long)ncol * (n_layer - cloud_top + 1);
   int blocks = (int)((cells + 255) / 256);
-  if (blocks > 152 * 16) blocks = 152 * 16;
+  if (blocks > 152 * 4) blocks = 152 * 4;
   if (blocks < 1) blocks = 1;
   cloud_range_kernel<<<blocks, 256, 0, st>>>(a);
   count_launch();
-  const int bs = gen_block(ncol);
-  cloud_gen_kernel<<<(ncol + bs - 1) / bs, bs, 0, st>>>(a);
-  count_launch();
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_generator(a, st);
   if (e != cudaSuccess) {
     snprintf(msg, len, "cloud_gen launch failed: %s", cudaGetErrorString(e));
     return SOCGPU_I_ABORT_CALCULATION;
@@ -369,10 +505,7 @@ int launch_cloud_gen_noalloc(int nd_layer, int cloud_top, int n_layer, int nd_pr
   }
   cloud_layer_range_kernel<<<1, 256, 0, st>>>(scratch, ncl > 0 ? ncl : 0, cloud_top, n_layer, range);
   count_launch();
-  const int bs = gen_block(ncol);
-  cloud_gen_kernel<<<(ncol + bs - 1) / bs, bs, 0, st>>>(a);
-  count_launch();
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_generator(a, st);
   if (e != cudaSuccess) {
     snprintf(msg, len, "cloud_gen launch failed: %s", cudaGetErrorString(e));
     return SOCGPU_I_ABORT_CALCULATION;
