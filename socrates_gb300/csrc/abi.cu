@@ -67,6 +67,38 @@ int launch_cloud_gen_noalloc(int nd_layer, int cloud_top, int n_layer, int nd_pr
 static std::atomic<long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
+// One pool per device, made on first use and kept for the process.
+static cudaMemPool_t scratch_pool() {
+  static std::mutex m;
+  static std::map<int, cudaMemPool_t> pools;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  std::lock_guard<std::mutex> lk(m);
+  auto it = pools.find(dev);
+  if (it != pools.end()) return it->second;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  unsigned long long keep = kScratchKeep;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  pools[dev] = pool;
+  return pool;
+}
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st) {
+  cudaMemPool_t pool = scratch_pool();
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
+}
+void scratch_free(void *p, cudaStream_t st) {
+  if (p) cudaFreeAsync(p, st);
+}
+void scratch_trim() {
+  cudaMemPool_t pool = scratch_pool();
+  if (pool) cudaMemPoolTrimTo(pool, 0);
+}
+
 void set_msg(char *msg, size_t len, const char *fmt, ...) {
   if (!msg || len == 0) return;
   va_list ap;
@@ -1586,7 +1618,7 @@ int upload_groups(std::vector<BatchGroup> &groups, char *&dbuf, std::vector<Flux
                   std::vector<long long *> &d_start, char *msg, size_t msg_len) {
   size_t bytes = 0;
   for (const BatchGroup &g : groups)
-    bytes += align256(sizeof(FluxParams) * g.n_items) + align256(sizeof(long long) * (g.n_items + 1));
+    bytes += align256(sizeof(FluxParams) * g.n_items) + align256(sizeof(long long) * (g.n_items + 1)) + align256(g.scratch);
   if (dbuf) { cudaFree(dbuf); dbuf = nullptr; }
   CUDA_TRY(cudaMalloc(&dbuf, std::max<size_t>(bytes, 256)));
   size_t off = 0;
@@ -1596,6 +1628,8 @@ int upload_groups(std::vector<BatchGroup> &groups, char *&dbuf, std::vector<Flux
     off += align256(sizeof(FluxParams) * g.n_items);
     long long *ds = (long long *)(dbuf + off);
     off += align256(sizeof(long long) * (g.n_items + 1));
+    for (int i = 0; i < g.n_items; ++i) g.items[i].region_scr = g.scratch ? dbuf + off : nullptr;
+    off += align256(g.scratch);
     CUDA_TRY(cudaMemcpy(di, g.items, sizeof(FluxParams) * g.n_items, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(ds, g.col_start, sizeof(long long) * (g.n_items + 1), cudaMemcpyHostToDevice));
     d_items.push_back(di);
@@ -1774,6 +1808,7 @@ int socgpu_spectrum_release(socgpu_spectrum_handle handle) {
   }
   cudaDeviceSynchronize();
   free_spectrum(*e);
+  scratch_trim();
   return SOCGPU_I_NORMAL;
 }
 

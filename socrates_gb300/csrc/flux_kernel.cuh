@@ -163,8 +163,7 @@ struct SmemLayout {
   size_t off_phf_nc, off_fwd_nc, off_c_ke, off_c_ks, off_c_ka, off_c_phf, off_c_fwd;
   size_t off_wcld, off_frac, off_csub;
   size_t off_aux, off_lkf, off_lki, off_sbf, off_sbj, off_kscr;
-  size_t off_ovl, off_reg, off_regd, off_nct, off_t0d, off_frr;
-  int reg_rows, regd_rows;            // rows per group of the region solves (two or three regions)
+  size_t off_ovl, off_nct, off_t0d, off_frr;
   size_t off_acc;
   // the column's FP64 inputs, fetched into shared memory ahead of staging
   // (offsets in doubles from off_acc, whose space they share); raw_on false
@@ -193,6 +192,22 @@ enum RegDRow { kRgB11, kRgB21, kRgB22, kRgG11, kRgG12, kRgG21, kRgG22, kRgH1, kR
                // elimination coefficients and its solar sources in FP64
                kRgB33 = kRegDRows, kRgG33, kRgH3, kRgSUV, kRgSDV, kRegDRows3 };
 
+// The rows of the region solves of a CTA, in global memory: a solve runs on
+// one thread, its 18 coefficient and 9 FP64 rows of n_layer + 1 values (25 and
+// 14 for three regions) interleaved by thread, so that the threads of a warp,
+// which walk the layers together, touch consecutive words.
+template <class T>
+struct Strided {
+  T *p;
+  int st;
+  __device__ __forceinline__ T &operator[](int i) const { return p[(size_t)i * st]; }
+};
+template <class R>
+__host__ __device__ inline size_t region_cta_bytes(const FluxParams &p) {
+  const size_t rows = p.triple ? kRegRows3 : kRegRows, rowsd = p.triple ? kRegDRows3 : kRegDRows;
+  return (size_t)p.region_rt * (p.n_layer + 1) * (rows * sizeof(R) + rowsd * sizeof(double));
+}
+
 // The layout of a column of batch p: nb bands staged at a time, n_groups
 // solve groups of P lanes, LP = P*CH layer slots.
 template <class R>
@@ -205,7 +220,6 @@ __host__ __device__ inline SmemLayout make_layout(const FluxParams &p, int LP, i
   size_t o = 0;
   auto take = [&](size_t elems) { size_t r = (o + 15) & ~(size_t)15; o = r + elems * sizeof(R); return r; };
   auto take_int = [&](size_t elems) { size_t r = (o + 15) & ~(size_t)15; o = r + elems * sizeof(int); return r; };
-  auto take_dbl = [&](size_t elems) { size_t r = (o + 15) & ~(size_t)15; o = r + elems * sizeof(double); return r; };
   s.off_p = take(LP);
   s.off_t = take(LP);
   s.off_mass = take(LP);
@@ -240,15 +254,11 @@ __host__ __device__ inline SmemLayout make_layout(const FluxParams &p, int LP, i
   s.off_sbj = p.n_sb > 0 ? take_int((size_t)p.n_sb * LP) : o;
   // per-group scratch row for k of per-term scaled absorbers
   s.off_kscr = p.term_scr ? take((size_t)n_groups * LP) : o;
-  // cloud regions: the column's interface coefficients and cloud top, and
-  // each group's rows for the serial two-region solve
+  // cloud regions: the column's interface coefficients and cloud top (the
+  // solves' rows lie in global memory, RegionScratch)
   const bool region = mcica && p.region;
   const bool triple = region && p.triple;
-  s.reg_rows = triple ? kRegRows3 : kRegRows;
-  s.regd_rows = triple ? kRegDRows3 : kRegDRows;
   s.off_ovl = region ? take((size_t)(triple ? 18 : 8) * (LP + 1)) : o;
-  s.off_reg = region ? take((size_t)n_groups * s.reg_rows * (LP + 1)) : o;
-  s.off_regd = region ? take_dbl((size_t)n_groups * s.regd_rows * (LP + 1)) : o;
   s.off_nct = region ? take_int(4) : o;
   // three regions: the stratiform and convective shares of each layer's
   // cloud (frac_region), by layer
@@ -435,8 +445,7 @@ struct FluxKernel {
     R *phf_nc, *fwd_nc, *c_ke, *c_ks, *c_ka, *c_phf, *c_fwd, *wcld, *frac, *csub;
     R *aux, *lkf, *sbf, *scr;    // scr: this thread's group's scratch row
     int *lki, *sbj;
-    R *ovl, *reg, *t0d, *frr;
-    double *regd;
+    R *ovl, *t0d, *frr;
     int *nct;
     Acc *acc;
     // the mixed kernels' depths and accumulators (flux_tau_kernel.cuh)
@@ -463,8 +472,7 @@ struct FluxKernel {
     s.lkf = (R *)(smem + l.off_lkf); s.lki = (int *)(smem + l.off_lki);
     s.sbf = (R *)(smem + l.off_sbf); s.sbj = (int *)(smem + l.off_sbj);
     s.scr = (R *)(smem + l.off_kscr) + (size_t)(threadIdx.x / P) * LP;
-    s.ovl = (R *)(smem + l.off_ovl); s.reg = (R *)(smem + l.off_reg); s.nct = (int *)(smem + l.off_nct);
-    s.regd = (double *)(smem + l.off_regd);
+    s.ovl = (R *)(smem + l.off_ovl); s.nct = (int *)(smem + l.off_nct);
     s.t0d = (R *)(smem + l.off_t0d);
     s.frr = (R *)(smem + l.off_frr);
     s.acc = (Acc *)(smem + l.off_acc);
@@ -725,15 +733,17 @@ struct FluxKernel {
     if (!S.raw)
       for (int q = threadIdx.x; q < n_groups * lay.acc_stride; q += nthreads) S.acc[q] = Acc(0);
     if (MCICA) stage_cloud_column(p, S, col);
-    if (MCICA && p.region) {
-      if (p.triple) stage_regions3(p, S, col, LP);
-      else stage_regions(p, S, col, LP);
-    }
     const int gid = threadIdx.x / P;
     const int r = threadIdx.x % P;
     const R sec0 = !p.zen_0 ? R(1) : (S.raw && S.r_alb > S.r_zen) ? raw_in<R>(S.raw[S.r_zen]) : load_in<R>(p.zen_0 + col);
     Acc *acc = S.acc + (size_t)gid * lay.acc_stride;
     __syncthreads();
+    // the overlap of the column's regions, by the last thread beside the
+    // staging of the bands (which does not read it)
+    if (MCICA && p.region) {
+      if (p.triple) stage_regions3(p, S, col, LP);
+      else stage_regions(p, S, col, LP);
+    }
 
     for (int bb = 0; bb < nb_all; bb += nbat) {
       const int nb = min(nbat, nb_all - bb);
@@ -761,12 +771,17 @@ struct FluxKernel {
       // first g-point of the batch and discards it.
       const int g_lo = p.bands[bstart].g_first;
       const int g_hi = p.bands[bstart + nb - 1].g_first + p.bands[bstart + nb - 1].g_count;
-      const int rounds = (g_hi - g_lo + n_groups - 1) / n_groups;
-      for (int rd = 0; rd < rounds; ++rd) {
-        int g = g_lo + rd * n_groups + gid;
-        const bool active = g < g_hi;
-        if (!active) g = g_lo;
-        solve_gpoint(p, S, col, g, bstart, max_abs, sec0, r, acc, lw, active);
+      if constexpr (MCICA)
+        if (p.region) solve_regions(p, S, g_lo, g_hi, bstart, sec0);
+      if constexpr (kFP64) {
+        // (in FP32 only cloud regions run here)
+        const int rounds = MCICA && p.region ? 0 : (g_hi - g_lo + n_groups - 1) / n_groups;
+        for (int rd = 0; rd < rounds; ++rd) {
+          int g = g_lo + rd * n_groups + gid;
+          const bool active = g < g_hi;
+          if (!active) g = g_lo;
+          solve_gpoint(p, S, col, g, bstart, max_abs, sec0, r, acc, lw, active);
+        }
       }
       __syncthreads();
       if (lw) {
@@ -1560,13 +1575,9 @@ struct FluxKernel {
     const R f_inc_down = bs[0], f_inc_dir = bs[1], alb_diff = bs[2], alb_dir = bs[3], dB_surf = bs[4];
 
     // the unscaled direct transmissions (i_direct_tau = ip_direct_noscaling)
-    R *t0d = (!lw && p.i_direct_tau == SOCGPU_IP_DIRECT_NOSCALING && !p.region)
+    R *t0d = (!lw && p.i_direct_tau == SOCGPU_IP_DIRECT_NOSCALING)
                  ? S.t0d + (size_t)(threadIdx.x / P) * LP : nullptr;
-    if constexpr (!kFP64 && P > 1) {
-      // the mixed kernels solve clear skies and McICA in optical-depth form
-      // (flux_tau_kernel.cuh); cloud regions come here
-      solve_region(p, g, bstart, sec0, r, lw, active);
-    } else if constexpr (!MCICA) {
+    if constexpr (!MCICA) {
       // the gas absorption of the lane's layers first, while few registers
       // are live, then the coefficients
       R kgv[CH];
@@ -1596,8 +1607,6 @@ struct FluxKernel {
         }
       solve_column(p, T, Rf, T0, c1, c2, om, r, L, lw, dB_b, dB2_b, f_inc_down, f_inc_dir,
                    alb_diff, alb_dir, dB_surf, w_g, acc, active, t0d);
-    } else if (p.region) {
-      solve_region(p, g, bstart, sec0, r, lw, active);
     } else {
       solve_mcica(p, S, col, gp, gt, bd, bi, b, r, L, lw, sec0, dB_b, dB2_b, f_inc_down, f_inc_dir,
                   alb_diff, alb_dir, dB_surf, w_g, acc, max_abs, active);
@@ -1623,11 +1632,9 @@ struct FluxKernel {
   // one (ovl rows 2 j + k) and of each lower region under each upper one
   // (rows 4 + 2 j + k).  The interfaces above the cloud top keep the identity.
   __device__ static void stage_regions(const FluxParams &p, const Smem &S, int col, int LP_) {
-    if (threadIdx.x != 0) return;
+    if (threadIdx.x != blockDim.x - 1) return;
     const int L = p.n_layer, ndp = p.nd_profile, ict = p.id_ct;
-    auto wc = [&](int i1) -> R {
-      return (i1 - 1 >= ict) ? load_in<R>(p.w_cloud + (size_t)col + (size_t)ndp * (size_t)(i1 - 1 - ict)) : R(0);
-    };
+    auto wc = [&](int i1) -> R { return S.wcld[slot(i1 - 1)]; };
     int nct = ict + 1;
     while (nct < L && !(wc(nct) > R(0))) ++nct;
     S.nct[0] = nct;
@@ -1668,11 +1675,9 @@ struct FluxKernel {
   // j (row 9 + 3 j + k).  The interfaces above the cloud top keep the
   // identity.
   __device__ static void stage_regions3(const FluxParams &p, const Smem &S, int col, int LP_) {
-    if (threadIdx.x != 0) return;
+    if (threadIdx.x != blockDim.x - 1) return;
     const int L = p.n_layer, ndp = p.nd_profile, ict = p.id_ct, ndc = p.nd_layer - ict;
-    auto wc = [&](int i1) -> R {
-      return (i1 - 1 >= ict) ? load_in<R>(p.w_cloud + (size_t)col + (size_t)ndp * (size_t)(i1 - 1 - ict)) : R(0);
-    };
+    auto wc = [&](int i1) -> R { return S.wcld[slot(i1 - 1)]; };
     int nct = ict + 1;
     while (nct < L && !(wc(nct) > R(0))) ++nct;
     S.nct[0] = nct;
@@ -1717,228 +1722,184 @@ struct FluxKernel {
     }
   }
 
-  // One g-point of a column in a clear and a cloudy region (mix_column.F90:
-  // 150-460).  The lanes of the group compute the clear coefficients and the
-  // frac_cloud-weighted coefficients of the cloud types (two_coeff_cloud.F90)
-  // of their layers, and the infra-red sources; lane 0 then runs the serial
-  // parts from the group's scratch rows: the direct beam through both regions
-  // (mixed_solar_source.F90), solver_mix_direct.F90 or
-  // solver_mix_direct_hogan.F90 and the back-substitution; the lanes add the
-  // level fluxes to the group's accumulators.
-  // Called out of line with scalars only, so that the McICA kernels it
-  // shares keep their registers: the shared-memory view, the g-point and
-  // the group's accumulators are rebuilt here as the column loop builds them.
-  __device__ static __noinline__ void solve_region(const FluxParams &p, int g, int bstart, R sec0, int r, bool lw,
-                                                   bool active) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int n_groups = blockDim.x / P, L = p.n_layer, max_abs = p.max_abs;
-    const SmemLayout lay = make_layout<R>(p, LP, P, p.band_batch, n_groups, MCICA);
-    const Smem S = bind(smem, lay);
+  // Clouds in two regions (mix_column.F90) or three (triple_column.F90): the
+  // solves of the staged bands' g-points, region_rt at a time.  Every thread
+  // of the CTA forms cells -- the clear coefficients and the frac_cloud-
+  // weighted ones of each cloudy region (two_coeff_cloud.F90,
+  // two_coeff_region.F90:230-440), and the infra-red sources weighted by the
+  // regions' areas -- lane = g-point; then one thread per g-point runs the
+  // serial parts: the direct beam through the regions (mixed_solar_source.F90,
+  // triple_solar_source.F90), solver_mix_direct.F90, its Hogan form or
+  // solver_triple_hogan.F90, and the back-substitution, in FP64; then the CTA
+  // sums the level fluxes over the g-points, in their order.
+  //
+  // The serial part is bound by the FP64 pipe (about 75 operations per cloudy
+  // layer, 76 cycles per warp instruction): it used to run on one lane of a
+  // group, and a warp instruction costs the same for one lane as for 32.
+  // Solar, two regions, 1025 x 70 x 48 on GB300: 12.94 ms with one lane per
+  // warp, 1.24 ms with a thread per g-point.
+  __device__ static void region_cell(const FluxParams &p, const Smem &S, R *X, int st, int g, int bstart, int i,
+                                     int nct, R sec0) {
+    constexpr bool lw = (SRC == SOCGPU_IP_INFRA_RED);
+    const int L = p.n_layer, max_abs = p.max_abs, s = slot(i);
     const GPoint &gp = p.gpoints[g];
-    const int b = gp.band, bi = b - bstart;
+    const int b = gp.band, bi = b - bstart, nc = p.n_condensed;
     const BandInfo &bd = p.bands[b];
-    const GasTerm gt = load_gas(gp, bd, max_abs);
-    const R *bs = S.bscal + bi * kBandScal;
-    const R w_g = kFP64 ? (R)(bs[5] * gp.weight) : (R)(bs[5] * gp.weight_f);
-    const R f_inc_down = bs[0], f_inc_dir = bs[1], alb_diff = bs[2], alb_dir = bs[3], dB_surf = bs[4];
-    const R *dB_b = S.dB + (size_t)bi * LP, *dB2_b = S.dB2 + (size_t)bi * LP;
-    const int nc = p.n_condensed;
-    const int gid = threadIdx.x / P;
-    Acc *acc = S.acc + (size_t)gid * lay.acc_stride;
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned gm = (P == 32) ? 0xffffffffu : (((1u << P) - 1u) << (lane & ~(unsigned)(P - 1)));
-    const R *kgt_b = S.kgt + (size_t)bi * LP, *kes_b = S.kes + (size_t)bi * LP;
-    const R *kabs_b = S.kabs + (size_t)bi * LP, *asym_b = S.asym + (size_t)bi * LP;
-    const R *fwd_b = S.fwd + (size_t)bi * LP, *amt_b = S.amt + (size_t)bi * max_abs * LP;
-    const R *phf_nc = S.phf_nc + (size_t)bi * LP, *fwd_nc = S.fwd_nc + (size_t)bi * LP;
-    const R *c_ke = S.c_ke + (size_t)bi * nc * LP, *c_ks = S.c_ks + (size_t)bi * nc * LP;
-    const R *c_ka = S.c_ka + (size_t)bi * nc * LP, *c_ph = S.c_phf + (size_t)bi * nc * LP;
-    const R *c_fw = S.c_fwd + (size_t)bi * nc * LP;
-    R *X = S.reg + (size_t)gid * lay.reg_rows * (LP + 1);
-    auto row = [&](int k) { return X + (size_t)k * (LP + 1); };
-    const int nct = S.nct[0];
+    auto at = [&](int k) -> R & { return X[((size_t)k * (L + 1) + i) * st]; };
+    const size_t q = (size_t)bi * LP + s, qb = (size_t)bi * nc * LP + s;
     const bool triple = p.triple;
-
-    R kgv[CH];
-    gas_k_lane(p, S, gt, gp, bd, amt_b, r, L, kgv);
-    R Tf[CH], Rff[CH], T0f[CH], c1f[CH], c2f[CH], omf[CH];
-    R Tc[CH], Rc[CH], T0c[CH], c1c[CH], c2c[CH], omc[CH];
-    // three regions: the convective region's coefficients are summed in its
-    // rows of the group's scratch (the stratiform region uses Tc..), so the
-    // McICA kernels this function shares keep their registers
-    R *VT = row(kRgVT), *VR = row(kRgVR), *VT0 = row(kRgVT0), *VC1 = row(kRgVC1), *VC2 = row(kRgVC2);
-    R *VOM = row(kRgVOM);
+    // the gas absorption (gas_optical_properties.F90:80-95)
+    R kg = R(0);
+    if (p.l_gas) {
+      const Lk lk = lk_of(S);
+      const int n_abs = min(gp.n_abs, max_abs);
+      for (int j = 0; j < n_abs; ++j) {
+        const R kj = kFP64 ? (R)gp.k[j] : (R)gp.kf[j];
+        const R *sc;
+        if constexpr (kFP64) sc = gp.term_scale[j]; else sc = gp.term_scale_f[j];
+        const R kal = term_k(p, lk, bd.gas[j], b, kj, sc, gp.lk_off[j], gp.iex[j],
+                             S.amt[((size_t)bi * max_abs + j) * LP + s], s, S.p[s], S.t[s]);
+        kg = (j == 0) ? kal : kg + kal;
+      }
+    }
     // the direct beam without delta-scaling (two_coeff.F90 trans_0_dir):
     // exp(-tau sec0) of the optical depth before rescaling, per region
     const bool dir_unscaled = !lw && p.i_direct_tau == SOCGPU_IP_DIRECT_NOSCALING;
-    auto t0_unscaled = [&](R kgt, R kg, R dm) -> R {
-      if constexpr (kFP64) return exp(-(kgt + kg) * dm * sec0);
-      else return expf(-(kgt + kg) * dm * sec0);
-    };
-#pragma unroll
-    for (int j = 0; j < CH; ++j) {
-      const int i = r * CH + j, s = j * P + r;
-      Tc[j] = R(0); Rc[j] = R(0); T0c[j] = R(0); c1c[j] = R(0); c2c[j] = R(0); omc[j] = R(0);
-      if (triple && i < L) { VT[i] = R(0); VR[i] = R(0); VT0[i] = R(0); VC1[i] = R(0); VC2[i] = R(0); VOM[i] = R(0); }
-      if (i < L && dir_unscaled) {
-        row(kRgFT0D)[i] = t0_unscaled(kgt_b[s], kgv[j], S.mass[s]); row(kRgCT0D)[i] = R(0);
-        if (triple) row(kRgVT0D)[i] = R(0);
-      }
-      if (i < L) {
-        cell_coef(p, kgt_b[s], kes_b[s], kabs_b[s], kgv[j], S.mass[s], asym_b[s], fwd_b[s], sec0,
-                  Tf[j], Rff[j], T0f[j], c1f[j], c2f[j], omf[j]);
-        if (S.wcld[s] > R(0)) {
-          for (int t = 0; t < p.n_cloud_type; ++t) {
-            const R fc = S.frac[(size_t)t * LP + s];
-            if (!(fc > R(0))) continue;
-            // the type's optical properties (grey_opt_prop.F90:980-1000,
-            // 1195-1240, 1475-1500; rescale_phase_fnc.F90)
-            R kgt = kgt_b[s], kes = kes_b[s], kab = kabs_b[s], fw = fwd_nc[s], ph = phf_nc[s];
-            for (int k = 0; k < nc; ++k) {
-              if (p.comp_type[k] - 1 != t) continue;
-              const size_t qk = (size_t)k * LP + s;
-              kgt = kgt + c_ke[qk]; kes = kes + c_ks[qk]; kab = kab + c_ka[qk];
-              fw = fw + c_fw[qk]; ph = ph + c_ph[qk];
-            }
-            R asym = ph, fwd = R(0);
-            if (kes > (R)kTiny64) {
-              const R inv = R(1) / kes;
-              if (p.l_rescale) {
-                fwd = fw * inv;
-                asym = (ph * inv - fwd) / (R(1) - fwd);
-              } else {
-                asym = ph * inv;
-              }
-            }
-            R tT, tR, tT0, t1, t2, tO;
-            cell_coef(p, kgt, kes, kab, kgv[j], S.mass[s], asym, fwd, sec0, tT, tR, tT0, t1, t2, tO);
-            if (triple && p.type_region[t] == 3) {
-              // a convective type (aggregate_cloud.F90:107-155)
-              VT[i] = VT[i] + fc * tT; VR[i] = VR[i] + fc * tR; VT0[i] = VT0[i] + fc * tT0;
-              if (dir_unscaled) row(kRgVT0D)[i] = row(kRgVT0D)[i] + fc * t0_unscaled(kgt, kgv[j], S.mass[s]);
-              VC1[i] = VC1[i] + fc * t1; VC2[i] = VC2[i] + fc * t2; VOM[i] = VOM[i] + fc * tO;
-            } else {
-              Tc[j] = Tc[j] + fc * tT; Rc[j] = Rc[j] + fc * tR; T0c[j] = T0c[j] + fc * tT0;
-              if (dir_unscaled) row(kRgCT0D)[i] = row(kRgCT0D)[i] + fc * t0_unscaled(kgt, kgv[j], S.mass[s]);
-              c1c[j] = c1c[j] + fc * t1; c2c[j] = c2c[j] + fc * t2; omc[j] = omc[j] + fc * tO;
-            }
-          }
-          if (triple) {
-            // each cloudy region's weighted sums over its share of the cloud
-            // (two_coeff_region.F90:383-440)
-            const R f2 = S.frr[i], f3 = S.frr[LP + i];
-            if (f2 > (R)kTiny64) {
-              const R inv = R(1) / f2;
-              Tc[j] = Tc[j] * inv; Rc[j] = Rc[j] * inv; T0c[j] = T0c[j] * inv;
-              c1c[j] = c1c[j] * inv; c2c[j] = c2c[j] * inv; omc[j] = omc[j] * inv;
-              if (dir_unscaled) row(kRgCT0D)[i] = row(kRgCT0D)[i] * inv;
-            }
-            if (f3 > (R)kTiny64) {
-              const R inv = R(1) / f3;
-              VT[i] = VT[i] * inv; VR[i] = VR[i] * inv; VT0[i] = VT0[i] * inv;
-              VC1[i] = VC1[i] * inv; VC2[i] = VC2[i] * inv; VOM[i] = VOM[i] * inv;
-              if (dir_unscaled) row(kRgVT0D)[i] = row(kRgVT0D)[i] * inv;
-            }
-          }
+    const R kgt0 = S.kgt[q], kes0 = S.kes[q], kab0 = S.kabs[q], dm = S.mass[s];
+    // region 0 the clear, 1 the (stratiform) cloudy, 2 the convective
+    R T[3] = {R(0), R(0), R(0)}, Rf[3] = {R(0), R(0), R(0)}, T0[3] = {R(0), R(0), R(0)};
+    R c1[3] = {R(0), R(0), R(0)}, c2[3] = {R(0), R(0), R(0)}, om[3] = {R(0), R(0), R(0)}, td[3] = {R(0), R(0), R(0)};
+    cell_coef(p, kgt0, kes0, kab0, kg, dm, S.asym[q], S.fwd[q], sec0, T[0], Rf[0], T0[0], c1[0], c2[0], om[0]);
+    if (dir_unscaled) td[0] = t0_unscaled(kgt0, kg, dm, sec0);
+    if (S.wcld[s] > R(0)) {
+      for (int t = 0; t < p.n_cloud_type; ++t) {
+        const R fc = S.frac[(size_t)t * LP + s];
+        if (!(fc > R(0))) continue;
+        // the type's optical properties (grey_opt_prop.F90:980-1000,
+        // 1195-1240, 1475-1500; rescale_phase_fnc.F90)
+        R kgt = kgt0, kes = kes0, kab = kab0, fw = S.fwd_nc[q], ph = S.phf_nc[q];
+        for (int k = 0; k < nc; ++k) {
+          if (p.comp_type[k] - 1 != t) continue;
+          const size_t qk = qb + (size_t)k * LP;
+          kgt = kgt + S.c_ke[qk]; kes = kes + S.c_ks[qk]; kab = kab + S.c_ka[qk];
+          fw = fw + S.c_fwd[qk]; ph = ph + S.c_phf[qk];
         }
-      } else {
-        Tf[j] = R(1); Rff[j] = R(0); T0f[j] = R(1); c1f[j] = R(0); c2f[j] = R(0); omf[j] = R(0);
-      }
-    }
-    if constexpr (SRC == SOCGPU_IP_SOLAR)
-      if (p.keqv) {
-        fold_direct(S, bi, max_abs, r, L, T0f, c2f);
-        fold_direct(S, bi, max_abs, r, L, T0c, c2c);
-        if (triple) {
-          // the same correction on the convective rows (fold_direct)
-          const R *a = S.aux + (size_t)bi * max_abs * LP;
-#pragma unroll
-          for (int j = 0; j < CH; ++j) {
-            const int i = r * CH + j, s = j * P + r;
-            if (i < L) {
-              const R fm1 = kFP64 ? a[s] - R(1) : a[s];
-              VC2[i] = VC2[i] + VT0[i] * fm1;
-              VT0[i] = kFP64 ? VT0[i] * a[s] : VT0[i] + VT0[i] * fm1;
-            }
-          }
-        }
-        if (dir_unscaled) {
-          // adjust_solar_ke on the unscaled beam too (mixed_solar_source.F90:130-140)
-          const R *a = S.aux + (size_t)bi * max_abs * LP;
-#pragma unroll
-          for (int j = 0; j < CH; ++j) {
-            const int i = r * CH + j, s = j * P + r;
-            if (i < L) {
-              const R f = kFP64 ? a[s] : R(1) + a[s];
-              row(kRgFT0D)[i] = row(kRgFT0D)[i] * f;
-              row(kRgCT0D)[i] = row(kRgCT0D)[i] * f;
-              if (triple) row(kRgVT0D)[i] = row(kRgVT0D)[i] * f;
-            }
-          }
-        }
-      }
-#pragma unroll
-    for (int j = 0; j < CH; ++j) {
-      const int i = r * CH + j, s = j * P + r;
-      if (i >= L) continue;
-      if (lw) {
-        // ir_source.F90:93-119 in each region, weighted by its area in the
-        // cloudy layers (mix_column.F90:185-230)
-        const R dB = dB_b[s];
-        R su, sd, suc, sdc, suv = R(0), sdv = R(0);
-        if (p.l_ir_source_quad) {
-          su = c1f[j] * dB + c2f[j] * dB2_b[s]; sd = -c1f[j] * dB + c2f[j] * dB2_b[s];
-          suc = c1c[j] * dB + c2c[j] * dB2_b[s]; sdc = -c1c[j] * dB + c2c[j] * dB2_b[s];
-          if (triple) { suv = VC1[i] * dB + VC2[i] * dB2_b[s]; sdv = -VC1[i] * dB + VC2[i] * dB2_b[s]; }
-        } else {
-          su = c1f[j] * dB; sd = -su; suc = c1c[j] * dB; sdc = -suc;
-          if (triple) { suv = VC1[i] * dB; sdv = -suv; }
-        }
-        if (i + 1 >= nct) {
-          const R wc = S.wcld[s], wf = R(1) - wc;
-          su = wf * su; sd = wf * sd;
-          if (triple) {
-            // the areas of the three regions (triple_column.F90:320-350)
-            const R a2 = wc * S.frr[i], a3 = wc * S.frr[LP + i];
-            suc = a2 * suc; sdc = a2 * sdc; suv = a3 * suv; sdv = a3 * sdv;
+        R asym = ph, fwd = R(0);
+        if (kes > (R)kTiny64) {
+          const R inv = R(1) / kes;
+          if (p.l_rescale) {
+            fwd = fw * inv;
+            asym = (ph * inv - fwd) / (R(1) - fwd);
           } else {
-            suc = wc * suc; sdc = wc * sdc;
+            asym = ph * inv;
           }
         }
-        c1f[j] = su; c2f[j] = sd; c1c[j] = suc; c2c[j] = sdc;
-        if (triple) { VC1[i] = suv; VC2[i] = sdv; }
-      }
-      row(kRgFT)[i] = Tf[j]; row(kRgFR)[i] = Rff[j]; row(kRgFT0)[i] = T0f[j];
-      row(kRgFC1)[i] = c1f[j]; row(kRgFC2)[i] = c2f[j]; row(kRgFOM)[i] = omf[j];
-      row(kRgCT)[i] = Tc[j]; row(kRgCR)[i] = Rc[j]; row(kRgCT0)[i] = T0c[j];
-      row(kRgCC1)[i] = c1c[j]; row(kRgCC2)[i] = c2c[j]; row(kRgCOM)[i] = omc[j];
-    }
-    __syncwarp(gm);
-    if (r == 0) {
-      double *Y = S.regd + (size_t)gid * lay.regd_rows * (LP + 1);
-      if (triple) region_serial3(p, S, X, Y, nct, L, lw, f_inc_down, f_inc_dir, alb_diff, alb_dir, dB_surf);
-      else region_serial(p, S, X, Y, nct, L, lw, f_inc_down, f_inc_dir, alb_diff, alb_dir, dB_surf);
-    }
-    __syncwarp(gm);
-    // accumulate the level fluxes and the layer divergence
-    const int L_acc = active ? L : -1;
-    Acc *acc_up = acc, *acc_dn = acc + (LP + 1), *acc_dir = acc + 2 * (LP + 1), *acc_div = acc + 3 * (LP + 1);
-    const R *fu = row(kRgFU), *fd = row(kRgFD), *fdir = row(kRgFDIR), *dv = row(kRgDIV);
-    if (r == 0 && active) {
-      acc_up[LP] += w_g * fu[0]; acc_dn[LP] += w_g * fd[0];
-      if (!lw) acc_dir[LP] += w_g * fdir[0];
-    }
+        R tT, tR, tT0, t1, t2, tO;
+        cell_coef(p, kgt, kes, kab, kg, dm, asym, fwd, sec0, tT, tR, tT0, t1, t2, tO);
+        const R tu = dir_unscaled ? t0_unscaled(kgt, kg, dm, sec0) : R(0);
+        // a convective type (aggregate_cloud.F90:107-155) or the cloudy region
+        const bool conv = triple && p.type_region[t] == 3;
 #pragma unroll
-    for (int j = 0; j < CH; ++j) {
-      const int i = r * CH + j, s = j * P + r;
-      if (i < L_acc) {
-        acc_up[s] += w_g * fu[i + 1];
-        acc_dn[s] += w_g * fd[i + 1];
-        if (!lw) acc_dir[s] += w_g * fdir[i + 1];
-        acc_div[s] += w_g * dv[i];
+        for (int k = 1; k < 3; ++k)
+          if (conv == (k == 2)) {
+            T[k] = T[k] + fc * tT; Rf[k] = Rf[k] + fc * tR; T0[k] = T0[k] + fc * tT0;
+            c1[k] = c1[k] + fc * t1; c2[k] = c2[k] + fc * t2; om[k] = om[k] + fc * tO;
+            td[k] = td[k] + fc * tu;
+          }
+      }
+      if (triple) {
+        // each cloudy region's weighted sums over its share of the cloud
+        // (two_coeff_region.F90:383-440)
+#pragma unroll
+        for (int k = 1; k < 3; ++k) {
+          const R f = S.frr[(size_t)(k - 1) * LP + i];
+          if (f > (R)kTiny64) {
+            const R inv = R(1) / f;
+            T[k] = T[k] * inv; Rf[k] = Rf[k] * inv; T0[k] = T0[k] * inv;
+            c1[k] = c1[k] * inv; c2[k] = c2[k] * inv; om[k] = om[k] * inv; td[k] = td[k] * inv;
+          }
+        }
       }
     }
-    __syncwarp(gm);
+    if constexpr (!lw)
+      if (p.keqv) {
+        // adjust_solar_ke (fold_direct; mixed_solar_source.F90:130-140)
+        const R a = S.aux[(size_t)bi * max_abs * LP + s], fm1 = kFP64 ? a - R(1) : a, f = kFP64 ? a : R(1) + a;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          c2[k] = c2[k] + T0[k] * fm1;
+          T0[k] = kFP64 ? T0[k] * a : T0[k] + T0[k] * fm1;
+          td[k] = td[k] * f;
+        }
+      }
+    if (lw) {
+      // ir_source.F90:93-119 in each region, weighted by its area in the
+      // cloudy layers (mix_column.F90:185-230, triple_column.F90:320-350)
+      const R dB = S.dB[q], wc = S.wcld[s];
+      const bool below = i + 1 >= nct;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        R su, sd;
+        if (p.l_ir_source_quad) {
+          su = c1[k] * dB + c2[k] * S.dB2[q]; sd = -c1[k] * dB + c2[k] * S.dB2[q];
+        } else {
+          su = c1[k] * dB; sd = -su;
+        }
+        if (below) {
+          const R area = k == 0 ? R(1) - wc : triple ? wc * S.frr[(size_t)(k - 1) * LP + i] : wc;
+          su = area * su; sd = area * sd;
+        }
+        c1[k] = su; c2[k] = sd;
+      }
+    }
+    at(kRgFT) = T[0]; at(kRgFR) = Rf[0]; at(kRgFT0) = T0[0]; at(kRgFC1) = c1[0]; at(kRgFC2) = c2[0]; at(kRgFOM) = om[0];
+    at(kRgCT) = T[1]; at(kRgCR) = Rf[1]; at(kRgCT0) = T0[1]; at(kRgCC1) = c1[1]; at(kRgCC2) = c2[1]; at(kRgCOM) = om[1];
+    if (dir_unscaled) { at(kRgFT0D) = td[0]; at(kRgCT0D) = td[1]; }
+    if (triple) {
+      at(kRgVT) = T[2]; at(kRgVR) = Rf[2]; at(kRgVT0) = T0[2]; at(kRgVC1) = c1[2]; at(kRgVC2) = c2[2]; at(kRgVOM) = om[2];
+      if (dir_unscaled) at(kRgVT0D) = td[2];
+    }
+  }
+
+  // g-points g_lo .. g_hi - 1; the sums go to the first group's accumulators.
+  __device__ static void solve_regions(const FluxParams &p, const Smem &S, int g_lo, int g_hi, int bstart, R sec0) {
+    constexpr bool lw = (SRC == SOCGPU_IP_INFRA_RED);
+    const int L = p.n_layer, st = p.region_rt, nct = S.nct[0], nt = blockDim.x;
+    R *X = (R *)((unsigned char *)p.region_scr + (size_t)blockIdx.x * region_cta_bytes<R>(p));
+    double *Y = (double *)(X + (size_t)(p.triple ? kRegRows3 : kRegRows) * (L + 1) * st);
+    // the serial threads: CTAs take the SM's schedulers in turn
+    const int t0 = ((int)threadIdx.x + nt - (int)(blockIdx.x * 64u) % nt) % nt;
+    for (int g0 = g_lo; g0 < g_hi; g0 += st) {
+      const int ng = min(st, g_hi - g0);
+      for (int q = threadIdx.x; q < L * st; q += nt) {
+        const int i = q / st, t = q - i * st;
+        if (t < ng) region_cell(p, S, X + t, st, g0 + t, bstart, i, nct, sec0);
+      }
+      __syncthreads();
+      for (int t = t0; t < ng; t += nt) {
+        const R *bs = S.bscal + (p.gpoints[g0 + t].band - bstart) * kBandScal;
+        if (p.triple) region_serial3(p, S, X + t, Y + t, st, nct, L, lw, bs[0], bs[1], bs[2], bs[3], bs[4]);
+        else region_serial(p, S, X + t, Y + t, st, nct, L, lw, bs[0], bs[1], bs[2], bs[3], bs[4]);
+      }
+      __syncthreads();
+      // a thread sums one level of one flux over the g-points
+      for (int q = threadIdx.x; q < 4 * (L + 1); q += nt) {
+        const int v = q / (L + 1), i = q - v * (L + 1);
+        if ((v == 2 && lw) || (v == 3 && i == L)) continue;
+        const int row = v == 0 ? kRgFU : v == 1 ? kRgFD : v == 2 ? kRgFDIR : kRgDIV;
+        const R *x = X + ((size_t)row * (L + 1) + i) * st;
+        R sum = R(0);
+        for (int t = 0; t < ng; ++t) {
+          const GPoint &gp = p.gpoints[g0 + t];
+          const R *bs = S.bscal + (gp.band - bstart) * kBandScal;
+          const R w = kFP64 ? (R)(bs[5] * gp.weight) : (R)(bs[5] * gp.weight_f);
+          sum += w * x[t];
+        }
+        // the divergence of layer i sits at its bottom level's slot
+        S.acc[(size_t)v * (LP + 1) + (v == 3 ? slot(i) : level_slot(i))] += sum;
+      }
+      __syncthreads();
+    }
   }
 
   // The serial part of the two-region solve, on one lane, in FP64 in every
@@ -1946,27 +1907,27 @@ struct FluxKernel {
   // solve_region leaves them; writes the level fluxes (diffuse in the
   // solar), the direct flux and the layer divergence.  Layers i are 0-based
   // here; interface i lies below layer i-1 (0: the top).
-  __device__ static __noinline__ void region_serial(const FluxParams &p, const Smem &S, R *X, double *Y, int nct,
+  __device__ static __noinline__ void region_serial(const FluxParams &p, const Smem &S, R *X, double *Y, int st, int nct,
                                                     int L, bool lw, R f_inc_down_r, R f_inc_dir_r, R alb_diff_r,
                                                     R alb_dir_r, R dB_surf_r) {
     using D = double;
-    auto row = [&](int k) { return X + (size_t)k * (LP + 1); };
-    auto drow = [&](int k) { return Y + (size_t)k * (LP + 1); };
+    auto row = [&](int k) { return Strided<R>{X + (size_t)k * (L + 1) * st, st}; };
+    auto drow = [&](int k) { return Strided<D>{Y + (size_t)k * (L + 1) * st, st}; };
     auto ov = [&](int m, int i) -> D { return (D)S.ovl[(size_t)m * (LP + 1) + i]; };
     const D f_inc_down = f_inc_down_r, f_inc_dir = f_inc_dir_r, alb_diff = alb_diff_r, alb_dir = alb_dir_r;
     const D dB_surf = dB_surf_r;
-    R *FT = row(kRgFT), *FR = row(kRgFR), *FT0 = row(kRgFT0), *FC1 = row(kRgFC1), *FC2 = row(kRgFC2);
-    R *CT = row(kRgCT), *CR = row(kRgCR), *CT0 = row(kRgCT0), *CC1 = row(kRgCC1), *CC2 = row(kRgCC2);
-    R *FOM = row(kRgFOM), *COM = row(kRgCOM);
-    D *B11 = drow(kRgB11), *B21 = drow(kRgB21), *B22 = drow(kRgB22), *G11 = drow(kRgG11), *G12 = drow(kRgG12);
-    D *G21 = drow(kRgG21), *G22 = drow(kRgG22), *H1 = drow(kRgH1), *H2 = drow(kRgH2);
-    R *FU = row(kRgFU), *FD = row(kRgFD), *FDIR = row(kRgFDIR), *DV = row(kRgDIV);
+    const Strided<R> FT = row(kRgFT), FR = row(kRgFR), FT0 = row(kRgFT0), FC1 = row(kRgFC1), FC2 = row(kRgFC2);
+    const Strided<R> CT = row(kRgCT), CR = row(kRgCR), CT0 = row(kRgCT0), CC1 = row(kRgCC1), CC2 = row(kRgCC2);
+    const Strided<R> FOM = row(kRgFOM), COM = row(kRgCOM);
+    const Strided<D> B11 = drow(kRgB11), B21 = drow(kRgB21), B22 = drow(kRgB22), G11 = drow(kRgG11), G12 = drow(kRgG12);
+    const Strided<D> G21 = drow(kRgG21), G22 = drow(kRgG22), H1 = drow(kRgH1), H2 = drow(kRgH2);
+    const Strided<R> FU = row(kRgFU), FD = row(kRgFD), FDIR = row(kRgFDIR), DV = row(kRgDIV);
     const bool hogan = p.solver_hogan;
     // the solar sources of each region in FP64 (mixed_solar_source.F90:
     // 95-250), held in four of the elimination rows until the elimination
     // (which reads a layer's sources before it writes that layer's row)
     // takes them over
-    D *SU = G21, *SD = G22, *SUC = G12, *SDC = B21;
+    const Strided<D> SU = G21, SD = G22, SUC = G12, SDC = B21;
     D bc = 0.0;
     if (!lw) {
       D f = f_inc_dir;
@@ -1992,7 +1953,7 @@ struct FluxKernel {
       if (p.i_direct_tau == SOCGPU_IP_DIRECT_NOSCALING) {
         // the direct flux without delta-scaling, which the outputs and the
         // ground's direct reflection take (mixed_solar_source.F90:200-240)
-        const R *FT0D = row(kRgFT0D), *CT0D = row(kRgCT0D);
+        const Strided<R> FT0D = row(kRgFT0D), CT0D = row(kRgCT0D);
         D fdd = f_inc_dir;
         for (int i1 = 1; i1 <= nct - 1; ++i1) { fdd = fdd * (D)FT0D[i1 - 1]; FDIR[i1] = (R)fdd; }
         D df = fdd, dc = 0.0;
@@ -2136,25 +2097,25 @@ struct FluxKernel {
   // 9 + 3 j + k); writes the level fluxes (diffuse in the solar), the direct
   // flux and the layer divergence.  Layers i are 0-based here; interface i
   // lies below layer i-1 (0: the top).
-  __device__ static __noinline__ void region_serial3(const FluxParams &p, const Smem &S, R *X, double *Y, int nct,
+  __device__ static __noinline__ void region_serial3(const FluxParams &p, const Smem &S, R *X, double *Y, int st, int nct,
                                                      int L, bool lw, R f_inc_down_r, R f_inc_dir_r, R alb_diff_r,
                                                      R alb_dir_r, R dB_surf_r) {
     using D = double;
-    auto row = [&](int k) { return X + (size_t)k * (LP + 1); };
-    auto drow = [&](int k) { return Y + (size_t)k * (LP + 1); };
+    auto row = [&](int k) { return Strided<R>{X + (size_t)k * (L + 1) * st, st}; };
+    auto drow = [&](int k) { return Strided<D>{Y + (size_t)k * (L + 1) * st, st}; };
     auto ov = [&](int m, int i) -> D { return (D)S.ovl[(size_t)m * (LP + 1) + i]; };
     const D f_inc_down = f_inc_down_r, f_inc_dir = f_inc_dir_r, alb_diff = alb_diff_r, alb_dir = alb_dir_r;
     const D dB_surf = dB_surf_r;
     // region k's rows: 0 the clear, 1 the stratiform, 2 the convective
-    R *T[3] = {row(kRgFT), row(kRgCT), row(kRgVT)}, *RR[3] = {row(kRgFR), row(kRgCR), row(kRgVR)};
-    R *T0[3] = {row(kRgFT0), row(kRgCT0), row(kRgVT0)}, *C1[3] = {row(kRgFC1), row(kRgCC1), row(kRgVC1)};
-    R *C2[3] = {row(kRgFC2), row(kRgCC2), row(kRgVC2)}, *OM[3] = {row(kRgFOM), row(kRgCOM), row(kRgVOM)};
-    D *B[3] = {drow(kRgB11), drow(kRgB22), drow(kRgB33)}, *G[3] = {drow(kRgG11), drow(kRgG22), drow(kRgG33)};
-    D *H[3] = {drow(kRgH1), drow(kRgH2), drow(kRgH3)};
+    const Strided<R> T[3] = {row(kRgFT), row(kRgCT), row(kRgVT)}, RR[3] = {row(kRgFR), row(kRgCR), row(kRgVR)};
+    const Strided<R> T0[3] = {row(kRgFT0), row(kRgCT0), row(kRgVT0)}, C1[3] = {row(kRgFC1), row(kRgCC1), row(kRgVC1)};
+    const Strided<R> C2[3] = {row(kRgFC2), row(kRgCC2), row(kRgVC2)}, OM[3] = {row(kRgFOM), row(kRgCOM), row(kRgVOM)};
+    const Strided<D> B[3] = {drow(kRgB11), drow(kRgB22), drow(kRgB33)}, G[3] = {drow(kRgG11), drow(kRgG22), drow(kRgG33)};
+    const Strided<D> H[3] = {drow(kRgH1), drow(kRgH2), drow(kRgH3)};
     // the solar sources of each region in FP64 (Hogan's form leaves the
     // coupling rows free)
-    D *SU[3] = {drow(kRgG21), drow(kRgG12), drow(kRgSUV)}, *SD[3] = {drow(kRgB21), drow(kRgH2), drow(kRgSDV)};
-    R *FU = row(kRgFU), *FD = row(kRgFD), *FDIR = row(kRgFDIR), *DV = row(kRgDIV);
+    const Strided<D> SU[3] = {drow(kRgG21), drow(kRgG12), drow(kRgSUV)}, SD[3] = {drow(kRgB21), drow(kRgH2), drow(kRgSDV)};
+    const Strided<R> FU = row(kRgFU), FD = row(kRgFD), FDIR = row(kRgFDIR), DV = row(kRgDIV);
     D base[3] = {0.0, 0.0, 0.0};
     if (!lw) {
       D f = f_inc_dir;
@@ -2182,7 +2143,7 @@ struct FluxKernel {
       if (p.i_direct_tau == SOCGPU_IP_DIRECT_NOSCALING) {
         // the direct flux without delta-scaling, which the outputs and the
         // ground's direct reflection take (triple_solar_source.F90:300-350)
-        const R *T0D[3] = {row(kRgFT0D), row(kRgCT0D), row(kRgVT0D)};
+        const Strided<R> T0D[3] = {row(kRgFT0D), row(kRgCT0D), row(kRgVT0D)};
         D fdd = f_inc_dir;
         for (int i1 = 1; i1 <= nct - 1; ++i1) { fdd = fdd * (D)T0D[0][i1 - 1]; FDIR[i1] = (R)fdd; }
         D db[3] = {fdd, 0.0, 0.0};
@@ -2627,11 +2588,21 @@ struct FluxKernel {
 // short chunks of the clear-sky kernels keep 4 CTAs of 256 threads (64
 // registers) per SM, which the shared memory of a 100-layer solar column
 // also allows; the McICA kernels would spill at 64 registers.
-constexpr int single_min_ctas(int ch, bool mcica) { return (ch <= 4 && !mcica) ? 4 : (ch <= 13 && !mcica ? 2 : 1); }
+constexpr int single_min_ctas(int ch, bool mcica, bool fp64) {
+  return !fp64 ? 2 : (ch <= 4 && !mcica) ? 4 : (ch <= 13 && !mcica ? 2 : 1);
+}
 
 template <class R, bool MIX, int P, int CH, bool NOSCAT, bool MCICA, int SRC>
-__global__ void __launch_bounds__(256, single_min_ctas(CH, MCICA)) flux_kernel(const __grid_constant__ FluxParams p) {
-  FluxKernel<R, MIX, P, CH, NOSCAT, MCICA, SRC>::run(p, blockIdx.x);
+__global__ void __launch_bounds__(256, single_min_ctas(CH, MCICA, sizeof(R) == 8)) flux_kernel(const __grid_constant__ FluxParams p) {
+  if constexpr (MCICA) {
+    // cloud regions: resident CTAs, each with its rows, stride over the columns
+    for (int col = blockIdx.x; col < p.n_profile; col += gridDim.x) {
+      if (col != blockIdx.x) __syncthreads();
+      FluxKernel<R, MIX, P, CH, NOSCAT, MCICA, SRC>::run(p, col);
+    }
+  } else {
+    FluxKernel<R, MIX, P, CH, NOSCAT, MCICA, SRC>::run(p, blockIdx.x);
+  }
 }
 
 // Persistent form over many column batches: items[i] describes one batch

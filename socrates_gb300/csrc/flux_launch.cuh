@@ -16,12 +16,32 @@ struct Shape { static constexpr int P = P_, CH = CH_; };
 template <class R, bool MCICA>
 constexpr bool tau_form(const FluxParams &p) { return sizeof(R) == 4 && !(MCICA && p.region); }
 
+constexpr int kRegionCtasPerSm = 2;
+
 // Shared memory the current device grants one CTA.
 inline int smem_limit() {
   int v = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   return v;
+}
+
+// Threads that solve a cloud-region column's g-points at a time: whole warps
+// for the calls of up to 64 g-points.
+inline int region_rt(const FluxParams &p) { return std::min(64, (p.g_end - p.g_begin + 15) / 16 * 16); }
+
+// Resident CTAs of a cloud-region launch: two to an SM keep the FP64 pipe of
+// its four schedulers busy, and more would only widen the rows' footprint.
+template <class K>
+int region_ctas(K kern, int threads, size_t bytes) {
+  int per_sm = 0, dev = 0, n_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, bytes) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    per_sm = 1;
+  }
+  return std::min(per_sm, kRegionCtasPerSm) * n_sm;
 }
 
 // One batch on the mixed kernel of shape S.
@@ -154,9 +174,20 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
     }
   }
   if (p.n_profile <= 0) return 0;
-  kern<<<p.n_profile, threads, lay.bytes, st>>>(q);
+  int grid = p.n_profile;
+  if (MCICA && p.region) {
+    grid = std::min(grid, region_ctas(kern, threads, lay.bytes));
+    q.region_rt = region_rt(p);
+    if (scratch_alloc(&q.region_scr, region_cta_bytes<R>(q) * grid, st) != cudaSuccess) {
+      cudaGetLastError();
+      snprintf(msg, len, "no device memory for the cloud regions' rows");
+      return SOCGPU_I_ABORT_CALCULATION;
+    }
+  }
+  kern<<<grid, threads, lay.bytes, st>>>(q);
   count_launch();
   cudaError_t e = cudaGetLastError();
+  if (MCICA && p.region) scratch_free(q.region_scr, st);
   if (e != cudaSuccess) {
     snprintf(msg, len, "flux kernel launch failed: %s", cudaGetErrorString(e));
     return SOCGPU_I_ABORT_CALCULATION;
@@ -240,6 +271,16 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
   g.smem = dyn;
   g.threads = warps * 32;
   g.grid = (int)std::min<long long>(g.total, (long long)per_sm * n_sm);
+  if (MCICA && g.n_items > 0 && g.items[0].region) {
+    // the resident CTAs' rows, sized for the widest item
+    g.grid = (int)std::min<long long>(g.total, (long long)std::min(per_sm, kRegionCtasPerSm) * n_sm);
+    size_t cta = 0;
+    for (int i = 0; i < g.n_items; ++i) {
+      g.items[i].region_rt = region_rt(g.items[i]);
+      cta = std::max(cta, region_cta_bytes<R>(g.items[i]));
+    }
+    g.scratch = cta * g.grid;
+  }
   }
   return 0;
 }

@@ -259,6 +259,7 @@ void launch_wave(socgpu_server_s &S, StreamSlot &sl) {
   size_t n_item = 0, n_start = 0;
   std::vector<BatchGroup> groups;
   std::vector<std::pair<size_t, size_t>> table_off;
+  std::vector<void *> scratch;
   for (auto &kv : classes) {
     BatchGroup g{};
     g.precision = std::get<0>(kv.first);
@@ -280,13 +281,27 @@ void launch_wave(socgpu_server_s &S, StreamSlot &sl) {
     const FluxVariant *v = find_variant(g.precision, g.mode, g.tile.lanes_per_solve);
     if (!v || v->prepare(g, msg, msg_len) != SOCGPU_I_NORMAL) {
       if (!v) snprintf(msg, msg_len, "no kernel built for %d lanes per solve", g.tile.lanes_per_solve);
+      for (void *q : scratch) scratch_free(q, st);
       fail_all(wave, SOCGPU_I_ERR_RANGE, msg);
       record_all(sl);
       return;
     }
     // one CTA per column (not the persistent grid): CTAs retire column by
-    // column, so higher-priority streams get SMs as they do
-    g.grid = (int)std::min<long long>(g.total, 0x7fffffffLL);
+    // column, so higher-priority streams get SMs as they do; cloud regions
+    // keep their resident CTAs, whose rows come from the library's pool
+    if (!g.scratch) g.grid = (int)std::min<long long>(g.total, 0x7fffffffLL);
+    if (g.scratch) {
+      void *rows = nullptr;
+      if (scratch_alloc(&rows, g.scratch, st) != cudaSuccess) {
+        cudaGetLastError();
+        for (void *q : scratch) scratch_free(q, st);
+        fail_all(wave, SOCGPU_I_ABORT_CALCULATION, "no device memory for the cloud regions' rows");
+        record_all(sl);
+        return;
+      }
+      scratch.push_back(rows);
+      for (int i = 0; i < g.n_items; ++i) g.items[i].region_scr = rows;
+    }
     groups.push_back(g);
     table_off.emplace_back(n_item, n_start);
     n_item += k;
@@ -306,6 +321,7 @@ void launch_wave(socgpu_server_s &S, StreamSlot &sl) {
     e = cudaLaunchKernel(g.kernel, dim3(g.grid), dim3(g.threads), args, g.smem, st);
     count_launch();
   }
+  for (void *q : scratch) scratch_free(q, st);
   if (e != cudaSuccess) {
     cudaGetLastError();
     fail_all(wave, SOCGPU_I_ABORT_CALCULATION, cudaGetErrorString(e));

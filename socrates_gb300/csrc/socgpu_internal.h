@@ -265,6 +265,10 @@ struct FluxParams {
   int triple;                        // three regions: clear, stratiform and convective (ip_cloud_triple)
   int type_region[4];                // the region (2 stratiform, 3 convective) of each 0-based cloud type
   TauLayout tau;                     // the mixed kernels' shared memory (set by the launcher)
+  // cloud regions: threads (g-points) that solve at a time, and the rows of
+  // the resident CTAs in global memory (set by the launcher)
+  int region_rt;
+  void *region_scr;
 };
 
 // Launch configuration chosen by the tuner.
@@ -288,6 +292,7 @@ struct BatchGroup {
   const void *kernel = nullptr;
   size_t smem = 0;
   int threads = 0, grid = 0;
+  size_t scratch = 0;                 // global scratch of the launch (cloud regions), for region_scr of every item
 };
 
 // Layers per lane (CH) instantiated for each precision and lane count P; a
@@ -370,5 +375,13 @@ inline bool phased_supported(const FluxParams &p) {
 }
 
 void count_launch();
+
+// Stream-ordered scratch of cloud-region launches, from a pool of the library
+// on the current device that keeps up to kScratchKeep bytes between launches
+// (socgpu_spectrum_release gives them back).
+constexpr size_t kScratchKeep = (size_t)512 << 20;
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st);
+void scratch_free(void *p, cudaStream_t st);
+void scratch_trim();
 
 }  // namespace socgpu
