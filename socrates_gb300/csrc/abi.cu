@@ -679,7 +679,7 @@ std::mutex g_tile_mutex;
 int g_tile[2][3][2] = {};   // [precision][mode][lanes, warps]
 std::map<std::tuple<int, int, int>, TileConfig> g_tuned;
 
-// Lanes per solve of the built-in tile.  FP64: 16 up to 128 layers, else 32.
+// Lanes per solve of the built-in tile.  FP64: 16 up to 144 layers, else 32.
 // Mixed clear skies: 8 up to 104 layers, 16 up to 144, else 32 -- few lanes
 // mean few scan steps per layer, as long as a lane's layers fit in 128
 // registers (measured on GB300, us: solar 10000 x 100 455 with 8 lanes, 485
@@ -689,7 +689,7 @@ std::map<std::tuple<int, int, int>, TileConfig> g_tuned;
 // 70 329 with 32, 342 with 16, 430 with 8): the lanes of a McICA warp then
 // share a subcolumn, and the minor absorbers' solves spread over more lanes.
 int built_in_lanes(int precision, int mode, int n_layer, bool keqv) {
-  if (precision != SOCGPU_PRECISION_MIXED) return n_layer <= 128 ? 16 : 32;
+  if (precision != SOCGPU_PRECISION_MIXED) return n_layer <= 144 ? 16 : 32;
   if (mode == 2 || keqv) return n_layer <= 64 ? 16 : 32;
   return n_layer <= 104 ? 8 : n_layer <= 144 ? 16 : 32;
 }

@@ -112,12 +112,22 @@ __device__ __forceinline__ Comp<R> comp_identity() {
   Comp<R> c; c.R1 = R(0); c.R2 = R(0); c.Td = R(1); c.Tu = R(1); c.Su = R(0); c.Sd = R(0); return c;
 }
 
+// Reciprocal for the solver's 1 - R rho: the hardware's approximation (some
+// 20 bits, not on the FP64 pipe) and two Newton steps, which leave it within
+// two units in the last place; a division takes twice the FP64 operations.
+__device__ __forceinline__ double recip(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = fma(fma(-x, r, 1.0), r, r);
+  return fma(fma(-x, r, 1.0), r, r);
+}
+
 // Stack A (above) on B (below).  Derived from the adding equations of
 // solver_homogen_direct: interface fluxes x (down) and y (up) satisfy
 // x = A.Sd + A.R2 y, y = B.Su + B.R1 x.
 template <class R>
 __device__ __forceinline__ Comp<R> stack(const Comp<R> &A, const Comp<R> &B) {
-  R D = R(1) / (R(1) - A.R2 * B.R1);
+  R D = recip(R(1) - A.R2 * B.R1);
   Comp<R> o;
   R dTd = D * A.Td, dTu = D * B.Tu;
   o.R1 = A.R1 + A.Tu * B.R1 * dTd;
@@ -129,36 +139,13 @@ __device__ __forceinline__ Comp<R> stack(const Comp<R> &A, const Comp<R> &B) {
   return o;
 }
 
-template <class R>
-__device__ __forceinline__ Comp<R> shfl_up_comp(const Comp<R> &c, int d, int width) {
-  Comp<R> o;
-  o.R1 = __shfl_up_sync(0xffffffffu, c.R1, d, width);
-  o.R2 = __shfl_up_sync(0xffffffffu, c.R2, d, width);
-  o.Td = __shfl_up_sync(0xffffffffu, c.Td, d, width);
-  o.Tu = __shfl_up_sync(0xffffffffu, c.Tu, d, width);
-  o.Su = __shfl_up_sync(0xffffffffu, c.Su, d, width);
-  o.Sd = __shfl_up_sync(0xffffffffu, c.Sd, d, width);
-  return o;
-}
-template <class R>
-__device__ __forceinline__ Comp<R> shfl_down_comp(const Comp<R> &c, int d, int width) {
-  Comp<R> o;
-  o.R1 = __shfl_down_sync(0xffffffffu, c.R1, d, width);
-  o.R2 = __shfl_down_sync(0xffffffffu, c.R2, d, width);
-  o.Td = __shfl_down_sync(0xffffffffu, c.Td, d, width);
-  o.Tu = __shfl_down_sync(0xffffffffu, c.Tu, d, width);
-  o.Su = __shfl_down_sync(0xffffffffu, c.Su, d, width);
-  o.Sd = __shfl_down_sync(0xffffffffu, c.Sd, d, width);
-  return o;
-}
-
 // ---------------------------------------------------------------------------
 // Shared-memory layout of one column (identical on host and device).  LP is
 // the padded layer count P*CH; level arrays hold LP+1 entries (slot LP is
 // level 0).
 struct SmemLayout {
   int LP, nb, max_abs, n_comp, n_sub, n_groups, acc_stride;
-  size_t off_p, off_t, off_mass, off_kgt, off_kes, off_kabs, off_asym, off_fwd, off_amt, off_bscal;
+  size_t off_p, off_t, off_mass, off_kgt, off_kes, off_kabs, off_asym, off_fwd, off_amt, off_ksi, off_bscal;
   size_t off_planck, off_dB, off_dB2;
   size_t off_phf_nc, off_fwd_nc, off_c_ke, off_c_ks, off_c_ka, off_c_phf, off_c_fwd;
   size_t off_wcld, off_frac, off_csub;
@@ -229,6 +216,8 @@ __host__ __device__ inline SmemLayout make_layout(const FluxParams &p, int LP, i
   s.off_asym = take((size_t)nb * LP);
   s.off_fwd = take((size_t)nb * LP);
   s.off_amt = take((size_t)nb * max_abs * LP);
+  // FP64, solar: ksi_0 of each cell (a division saved per g-point)
+  s.off_ksi = (sizeof(R) == 8 && !lw) ? take((size_t)nb * LP) : o;
   s.off_bscal = take((size_t)nb * kBandScal);
   s.off_planck = lw ? take((size_t)nb * (LP + 1)) : o;
   s.off_dB = lw ? take((size_t)nb * LP) : o;
@@ -389,7 +378,8 @@ struct FluxKernel {
   // kgt/kes/kabs: grey extinction, scattering, absorption; asym/fwd: g' and f.
   __device__ static __forceinline__ void cell_coef(const FluxParams &p, R kgt, R kes, R kabs, R kgas,
                                                    R dm, R asym, R fwd, R sec0,
-                                                   R &T, R &Rf, R &T0, R &c1, R &c2, R &omtr) {
+                                                   R &T, R &Rf, R &T0, R &c1, R &c2, R &omtr,
+                                                   const R *ksi = nullptr) {
     if constexpr (kFP64) {
       // single_scattering.F90:119-164, rescale_tau_omega.F90:73-80
       double tau, om;
@@ -409,7 +399,7 @@ struct FluxKernel {
         om = om * (1.0 - fwd) / (1.0 - om * fwd);
       }
       Coef c = NOSCAT ? fast_lw_ref(p.l_ir_source_quad, tau)
-                      : two_coeff_ref(SRC, p.i_2stream, p.l_ir_source_quad, asym, om, tau, sec0);
+                      : two_coeff_ref(SRC, p.i_2stream, p.l_ir_source_quad, asym, om, tau, sec0, ksi);
       T = c.T; Rf = c.R; T0 = c.T0; c1 = c.c1; c2 = c.c2; omtr = R(0);
     } else {
       float tau, om, omc;
@@ -441,7 +431,7 @@ struct FluxKernel {
   }
 
   struct Smem {
-    R *p, *t, *mass, *kgt, *kes, *kabs, *asym, *fwd, *amt, *bscal, *planck, *dB, *dB2;
+    R *p, *t, *mass, *kgt, *kes, *kabs, *asym, *fwd, *amt, *ksi, *bscal, *planck, *dB, *dB2;
     R *phf_nc, *fwd_nc, *c_ke, *c_ks, *c_ka, *c_phf, *c_fwd, *wcld, *frac, *csub;
     R *aux, *lkf, *sbf, *scr;    // scr: this thread's group's scratch row
     int *lki, *sbj;
@@ -462,6 +452,7 @@ struct FluxKernel {
     s.p = (R *)(smem + l.off_p); s.t = (R *)(smem + l.off_t); s.mass = (R *)(smem + l.off_mass);
     s.kgt = (R *)(smem + l.off_kgt); s.kes = (R *)(smem + l.off_kes); s.kabs = (R *)(smem + l.off_kabs);
     s.asym = (R *)(smem + l.off_asym); s.fwd = (R *)(smem + l.off_fwd); s.amt = (R *)(smem + l.off_amt);
+    s.ksi = (R *)(smem + l.off_ksi);
     s.bscal = (R *)(smem + l.off_bscal);
     s.planck = (R *)(smem + l.off_planck); s.dB = (R *)(smem + l.off_dB); s.dB2 = (R *)(smem + l.off_dB2);
     s.phf_nc = (R *)(smem + l.off_phf_nc); s.fwd_nc = (R *)(smem + l.off_fwd_nc);
@@ -752,6 +743,9 @@ struct FluxKernel {
       if (MCICA) stage_cloud_bands(p, S, col, bstart, nb);
       __syncthreads();
       stage_boundary(p, S, col, bstart, nb, lw);
+      if constexpr (kFP64 && !lw)
+        for (int q = threadIdx.x; q < nb * LP; q += nthreads)
+          if (layer_of_slot(q % LP) < L) S.ksi[q] = ksi0_ref(p.i_2stream, S.asym[q], sec0);
       __syncthreads();
       if (S.raw) {
         // the raw inputs are consumed: their space becomes the accumulators
@@ -1588,7 +1582,7 @@ struct FluxKernel {
         const int i = r * CH + j, s = j * P + r;
         if (i < L) {
           cell_coef(p, kgt_b[s], kes_b[s], kabs_b[s], kgv[j], S.mass[s], asym_b[s], fwd_b[s], sec0,
-                    T[j], Rf[j], T0[j], c1[j], c2[j], om[j]);
+                    T[j], Rf[j], T0[j], c1[j], c2[j], om[j], S.ksi + (size_t)bi * LP + s);
         } else {
           T[j] = R(1); Rf[j] = R(0); T0[j] = R(1); c1[j] = R(0); c2[j] = R(0); om[j] = R(0);
         }
@@ -2308,7 +2302,7 @@ struct FluxKernel {
           }
           if (!cloudy) {
             cell_coef(p, kgt_b[s], kes_b[s], kabs_b[s], kg, S.mass[s], asym_b[s], fwd_b[s], sec0,
-                      T[jj], Rf[jj], T0[jj], c1[jj], c2[jj], om[jj]);
+                      T[jj], Rf[jj], T0[jj], c1[jj], c2[jj], om[jj], S.ksi + (size_t)bi * LP + s);
             if (t0d) t0d[s] = t0_unscaled(kgt_b[s], kg, S.mass[s], sec0);
           } else {
             // mcica_sample.F90:472-700 then mcica_column.F90:336-470: each
@@ -2504,57 +2498,53 @@ struct FluxKernel {
     }
 
     // --- adding method (solver_homogen_direct.F90:94-131), eliminated from
-    // the top down: at each level F_dn = rho F_up + sig, and across layer j
-    // F_up(top) = a_j F_up(bottom) + b_j.  The chunks' states from above come
-    // from a prefix scan of their layer composites; the upward fluxes at the
-    // chunk bottoms from a suffix scan of the chunks' affine maps (a, b).
-    // the chunk's composite, stacked pairwise (a tree of depth log2 CH, so
-    // that the divisions of independent pairs overlap)
-    Comp<R> cc;
-    {
-      Comp<R> lv[CH];
+    // the top down.  The lane stacks its layers into one composite cc and
+    // keeps, per layer j with the stack `cc above j` before it,
+    //   F_up(top of j) = a_j F_up(bottom of j) + e_j F_dn(chunk top) + g_j
+    //   F_dn(top of j) = r_j F_up(top of j) + t_j F_dn(chunk top) + s_j
+    // so each layer costs one reciprocal (the FP64 pipe bounds this kernel:
+    // stacking the chunk as a tree and eliminating it again took two).  A
+    // prefix scan of the composites gives F_dn = rho F_up + sig at the chunk
+    // tops, a suffix scan of the chunks' affine maps F_up at their bottoms.
+    // Padding layers (T = 1, R = 0, no sources) are the identity.
+    Comp<R> cc = comp_identity<R>();
 #pragma unroll
-      for (int j = 0; j < CH; ++j) {
-        lv[j].R1 = Rf[j]; lv[j].R2 = Rf[j]; lv[j].Td = T[j]; lv[j].Tu = T[j]; lv[j].Su = c1[j]; lv[j].Sd = c2[j];
-      }
-#pragma unroll
-      for (int w = 1; w < CH; w <<= 1)
-#pragma unroll
-        for (int j = 0; j + w < CH; j += 2 * w) lv[j] = stack(lv[j], lv[j + w]);
-      cc = lv[0];
+    for (int j = 0; j < CH; ++j) {
+      const R su = c1[j], sd = c2[j], d = recip(R(1) - cc.R2 * Rf[j]);
+      const R a = T[j] * d, e = d * Rf[j] * cc.Td, g = d * (Rf[j] * cc.Sd + su);
+      const R r2 = Rf[j] + T[j] * cc.R2 * a, sn = sd + a * (cc.Sd + cc.R2 * su);
+      T0[j] = cc.R2; om[j] = cc.Td; c2[j] = cc.Sd;
+      cc.R1 = cc.R1 + cc.Td * e;
+      cc.Su = cc.Su + cc.Td * g;
+      cc.R2 = r2; cc.Sd = sn;
+      cc.Td = cc.Td * a;
+      T[j] = a; Rf[j] = e; c1[j] = g;
     }
+    cc.Tu = cc.Td;           // a stack of symmetric layers transmits alike both ways
     // above: inclusive prefix C_0 .. C_r, then the exclusive one
     Comp<R> pre = cc;
 #pragma unroll
     for (int d = 1; d < P; d <<= 1) {
-      Comp<R> y = shfl_up_comp(pre, d, P);
+      Comp<R> y;
+      y.R1 = __shfl_up_sync(0xffffffffu, pre.R1, d, P);
+      y.R2 = __shfl_up_sync(0xffffffffu, pre.R2, d, P);
+      y.Td = y.Tu = __shfl_up_sync(0xffffffffu, pre.Td, d, P);
+      y.Su = __shfl_up_sync(0xffffffffu, pre.Su, d, P);
+      y.Sd = __shfl_up_sync(0xffffffffu, pre.Sd, d, P);
       if (r >= d) pre = stack(y, pre);
     }
-    Comp<R> ex = shfl_up_comp(pre, 1, P);
-    R rho, sig;            // the state at the top of this chunk
+    R rho = __shfl_up_sync(0xffffffffu, pre.R2, 1, P);      // the state at the top of this chunk
+    R sig = __shfl_up_sync(0xffffffffu, pre.Sd + pre.Td * f_inc_down, 1, P);
     if (r == 0) { rho = R(0); sig = f_inc_down; }
-    else { rho = ex.R2; sig = ex.Sd + ex.Td * f_inc_down; }
-    // elimination through the chunk.  The arrays now hold, per layer,
-    // a (T), b (Rf) and the state at its top, rho (c1) and sig (c2);
-    // F_up(chunk top) = A F_up(chunk bottom) + B.  Padding layers (T = 1,
-    // R = 0, no sources) are the identity.
-    R A = R(1), B = R(0);
-#pragma unroll
-    for (int j = 0; j < CH; ++j) {
-      const R q = R(1) / (R(1) - Rf[j] * rho);
-      const R a = T[j] * q;
-      const R b = (Rf[j] * sig + c1[j]) * q;
-      const R rho_n = Rf[j] + (T[j] * T[j] * rho) * q;     // T^2 rho formed beside the division
-      const R sig_n = c2[j] + a * (sig + rho * c1[j]);
-      T[j] = a; Rf[j] = b; c1[j] = rho; c2[j] = sig;
-      B = B + A * b; A = A * a;
-      rho = rho_n; sig = sig_n;
-    }
+    // F_up(chunk top) = A F_up(chunk bottom) + B
+    const R q1 = recip(R(1) - cc.R1 * rho);
+    R A = cc.Td * q1, B = (cc.Su + cc.R1 * sig) * q1;
     // the surface closes the last chunk: F_up = alb F_dn + src_ground with
-    // F_dn = rho F_up + sig; that chunk's map becomes the constant F_up(top)
+    // F_dn = rb F_up + sb; that chunk's map becomes the constant F_up(top)
     R fu_surf = R(0);
     if (r == P - 1) {
-      fu_surf = (alb_diff * sig + src_ground) / (R(1) - alb_diff * rho);
+      const R rb = cc.R2 + cc.Td * rho * A, sb = cc.Sd + cc.Td * (rho * B + sig);
+      fu_surf = (alb_diff * sb + src_ground) / (R(1) - alb_diff * rb);
       B = A * fu_surf + B; A = R(0);
     }
     // suffix scan of the affine maps: F_up at the top of every chunk
@@ -2565,14 +2555,15 @@ struct FluxKernel {
     }
     R fu = __shfl_down_sync(0xffffffffu, B, 1, P);     // F_up at the bottom of this chunk
     if (r == P - 1) fu = fu_surf;
-    R fd = rho * fu + sig;
+    const R fdt = rho * B + sig;                       // F_dn at its top
+    R fd = cc.R2 * fu + (cc.Td * fdt + cc.Sd);         // F_dn at its bottom
     // back-substitution from the chunk bottom up, accumulating the level
     // below each layer and the layer's divergence
 #pragma unroll
     for (int j = CH - 1; j >= 0; --j) {
       const int i = r * CH + j, s = j * P + r;
-      const R fu_top = T[j] * fu + Rf[j];
-      const R fd_top = c1[j] * fu_top + c2[j];
+      const R fu_top = T[j] * fu + (Rf[j] * fdt + c1[j]);
+      const R fd_top = T0[j] * fu_top + (om[j] * fdt + c2[j]);
       if (i < L_acc) {
         acc_up[s] += w * fu;
         acc_dn[s] += w * fd;
@@ -2584,13 +2575,11 @@ struct FluxKernel {
   }
 };
 
-// Resident CTAs asked of the register allocator for the single-batch kernel:
-// short chunks of the clear-sky kernels keep 4 CTAs of 256 threads (64
-// registers) per SM, which the shared memory of a 100-layer solar column
-// also allows; the McICA kernels would spill at 64 registers.
-constexpr int single_min_ctas(int ch, bool mcica, bool fp64) {
-  return !fp64 ? 2 : (ch <= 4 && !mcica) ? 4 : (ch <= 13 && !mcica ? 2 : 1);
-}
+// Resident CTAs of 256 threads asked of the register allocator: two (128
+// registers) for cloud regions in FP32 and for FP64 chunks up to 6 layers
+// under clear skies, which fit without spills; one else.  The FP64 pipe bounds
+// these kernels: 8 warps an SM keep it busy.
+constexpr int single_min_ctas(int ch, bool mcica, bool fp64) { return !fp64 || (ch <= 6 && !mcica) ? 2 : 1; }
 
 template <class R, bool MIX, int P, int CH, bool NOSCAT, bool MCICA, int SRC>
 __global__ void __launch_bounds__(256, single_min_ctas(CH, MCICA, sizeof(R) == 8)) flux_kernel(const __grid_constant__ FluxParams p) {
@@ -2610,15 +2599,12 @@ __global__ void __launch_bounds__(256, single_min_ctas(CH, MCICA, sizeof(R) == 8
 // indices col_start[i] .. col_start[i+1]-1, one per column.  Each CTA strides
 // over the work indices, finds the batch by binary search and keeps the
 // batch's parameters in shared memory while consecutive indices stay in it.
-// Resident CTAs the batched kernel asks the register allocator for: its
-// parameters sit in shared memory, not in the constant bank, so without a
-// bound it keeps about twice the registers of flux_kernel (measured with
-// -Xptxas -v: 3 CTAs of 256 threads fit without spills up to 4 layers per
-// lane).
-constexpr int batched_min_ctas(int ch) { return ch <= 4 ? 3 : (ch <= 9 ? 2 : 1); }
+// The batched kernel's parameters sit in shared memory, not in the constant
+// bank, which costs it registers.
+constexpr int batched_min_ctas(int ch, bool mcica, bool fp64) { return !fp64 || (ch <= 5 && !mcica) ? 2 : 1; }
 
 template <class R, bool MIX, int P, int CH, bool NOSCAT, bool MCICA, int SRC>
-__global__ void __launch_bounds__(256, batched_min_ctas(CH))
+__global__ void __launch_bounds__(256, batched_min_ctas(CH, MCICA, sizeof(R) == 8))
 flux_kernel_batched(const FluxParams *__restrict__ items, const long long *__restrict__ col_start, int n_items,
                     long long total) {
   __shared__ __align__(16) FluxParams sp;

@@ -16,7 +16,7 @@ struct Shape { static constexpr int P = P_, CH = CH_; };
 template <class R, bool MCICA>
 constexpr bool tau_form(const FluxParams &p) { return sizeof(R) == 4 && !(MCICA && p.region); }
 
-constexpr int kRegionCtasPerSm = 2;
+constexpr int kRegionCtasPerSm = 4, kRegionWarps = 4;
 
 // Shared memory the current device grants one CTA.
 inline int smem_limit() {
@@ -30,8 +30,8 @@ inline int smem_limit() {
 // for the calls of up to 64 g-points.
 inline int region_rt(const FluxParams &p) { return std::min(64, (p.g_end - p.g_begin + 15) / 16 * 16); }
 
-// Resident CTAs of a cloud-region launch: two to an SM keep the FP64 pipe of
-// its four schedulers busy, and more would only widen the rows' footprint.
+// Resident CTAs of a cloud-region launch: four of four warps to an SM (solar,
+// 1025 x 70 x 48: 904 us; two of eight warps 1232, four of two 987).
 template <class K>
 int region_ctas(K kern, int threads, size_t bytes) {
   int per_sm = 0, dev = 0, n_sm = 0;
@@ -149,7 +149,7 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   // widest band batch (then most warps) whose staging fits in shared memory
-  int warps = cfg.warps_per_cta, batch = nb;
+  int warps = MCICA && p.region ? std::min(cfg.warps_per_cta, kRegionWarps) : cfg.warps_per_cta, batch = nb;
   SmemLayout lay{};
   for (;;) {
     lay = make_layout<R>(p, S::P * S::CH, S::P, batch, warps * 32 / S::P, MCICA,
@@ -212,7 +212,8 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-  const int warps = g.tile.warps_per_cta;
+  const bool region = MCICA && g.n_items > 0 && g.items[0].region;
+  const int warps = region ? std::min(g.tile.warps_per_cta, kRegionWarps) : g.tile.warps_per_cta;
   const int n_groups = warps * 32 / S::P;
   auto bytes_of = [&](const FluxParams &p, int batch) {
     return make_layout<R>(p, S::P * S::CH, S::P, batch, n_groups, MCICA,
@@ -271,7 +272,7 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
   g.smem = dyn;
   g.threads = warps * 32;
   g.grid = (int)std::min<long long>(g.total, (long long)per_sm * n_sm);
-  if (MCICA && g.n_items > 0 && g.items[0].region) {
+  if (region) {
     // the resident CTAs' rows, sized for the widest item
     g.grid = (int)std::min<long long>(g.total, (long long)std::min(per_sm, kRegionCtasPerSm) * n_sm);
     size_t cta = 0;

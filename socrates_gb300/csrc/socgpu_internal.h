@@ -301,7 +301,7 @@ struct BatchGroup {
 #define SOCGPU_CHUNKS_MIXED_8  5, 8, 9, 11, 13, 18
 #define SOCGPU_CHUNKS_MIXED_16 3, 4, 5, 7, 9, 16
 #define SOCGPU_CHUNKS_MIXED_32 3, 4, 5, 8, 16
-#define SOCGPU_CHUNKS_FP64_16  4, 8, 16
+#define SOCGPU_CHUNKS_FP64_16  3, 4, 5, 6, 7, 8, 9, 16
 #define SOCGPU_CHUNKS_FP64_32  4, 5, 8, 16
 
 // The chunks of (precision, lanes) in ascending order; returns their count

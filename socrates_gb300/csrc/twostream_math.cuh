@@ -54,8 +54,14 @@ __device__ __forceinline__ void sum_diff_ref(int scheme, double om, double g, do
 }
 
 // ---- full two-stream coefficients, reference form -------------------------
+// ksi_0 of the solar coefficients, which does not depend on the g-point.
+__device__ __forceinline__ double ksi0_ref(int scheme, double g, double sec0) {
+  return (scheme == SOCGPU_IP_DISCRETE_ORD) ? kRoot3 * g / sec0 : 1.5 * g / sec0;
+}
+// ksi_at: the staged ksi_0 of the cell, or null to form it here.
 __device__ __forceinline__ Coef two_coeff_ref(int isolir, int scheme, int l_quad,
-                                              double g, double om, double tau, double sec0) {
+                                              double g, double om, double tau, double sec0,
+                                              const double *ksi_at = nullptr) {
   Coef c;
   double sum, diff;
   sum_diff_ref(scheme, om, g, sum, diff);
@@ -68,7 +74,7 @@ __device__ __forceinline__ Coef two_coeff_ref(int isolir, int scheme, int l_quad
       diff = (1.0 + tol_perturb) * diff;
       lambda = (1.0 + tol_perturb) * lambda;
     }
-    double ksi0 = (scheme == SOCGPU_IP_DISCRETE_ORD) ? kRoot3 * g / sec0 : 1.5 * g / sec0;
+    const double ksi0 = ksi_at ? *ksi_at : ksi0_ref(scheme, g, sec0);
     double factor = 0.5 * om * sec0 / ((lambda - sec0) * (lambda + sec0));
     gam_up = factor * (sum - sec0 - ksi0 * (diff - sec0));
     gam_dn = factor * (sum + sec0 + ksi0 * (diff + sec0));
