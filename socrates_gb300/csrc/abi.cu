@@ -680,17 +680,17 @@ int g_tile[2][3][2] = {};   // [precision][mode][lanes, warps]
 std::map<std::tuple<int, int, int>, TileConfig> g_tuned;
 
 // Lanes per solve of the built-in tile.  FP64: 16 up to 144 layers, else 32.
-// Mixed clear skies: 8 up to 104 layers, 16 up to 144, else 32 -- few lanes
-// mean few scan steps per layer, as long as a lane's layers fit in 128
-// registers (measured on GB300, us: solar 10000 x 100 455 with 8 lanes, 485
-// with 16, 627 with 32; scattering long wave 3001 x 137 377 with 16, 443 with
-// 32, 575 with 8).  McICA and equivalent extinction: 16 up to 64 layers, else
-// 32 (solar McICA 8000 x 85 1252 with 32, 1453 with 8; GA9 short wave 2000 x
-// 70 329 with 32, 342 with 16, 430 with 8): the lanes of a McICA warp then
-// share a subcolumn, and the minor absorbers' solves spread over more lanes.
-int built_in_lanes(int precision, int mode, int n_layer, bool keqv) {
+// Mixed: 8 up to 104 layers, 16 up to 144, else 32 -- few lanes mean few scan
+// steps per layer, as long as a lane's layers fit in 128 registers (measured on
+// GB300, us: solar 10000 x 100 458 with 8 lanes, 497 with 16, 638 with 32;
+// scattering long wave 3001 x 137 367 with 16, 422 with 32, 588 with 8; solar
+// McICA 8000 x 85 830, 932, 978 with 8, 16, 32; long-wave McICA 4000 x 60 593
+// with 8, 640 with 16).  Equivalent extinction: 16 up to 64 layers, else 32
+// (GA9 short wave 2000 x 70 284 with 32, 288 with 16, 343 with 8): the minor
+// absorbers' solves then spread over more lanes.
+int built_in_lanes(int precision, int n_layer, bool keqv) {
   if (precision != SOCGPU_PRECISION_MIXED) return n_layer <= 144 ? 16 : 32;
-  if (mode == 2 || keqv) return n_layer <= 64 ? 16 : 32;
+  if (keqv) return n_layer <= 64 ? 16 : 32;
   return n_layer <= 104 ? 8 : n_layer <= 144 ? 16 : 32;
 }
 
@@ -702,9 +702,9 @@ int built_in_warps(int precision, bool keqv, int nd_profile) {
 }
 
 // The built-in scan tile, with the smallest chunk covering the column.
-TileConfig scan_tile(int precision, int mode, int n_layer, bool keqv, int nd_profile) {
+TileConfig scan_tile(int precision, int n_layer, bool keqv, int nd_profile) {
   TileConfig t{};
-  t.lanes_per_solve = built_in_lanes(precision, mode, n_layer, keqv);
+  t.lanes_per_solve = built_in_lanes(precision, n_layer, keqv);
   t.warps_per_cta = built_in_warps(precision, keqv, nd_profile);
   while (t.lanes_per_solve < 32 && smallest_chunk(precision, t.lanes_per_solve, n_layer) == 0) t.lanes_per_solve *= 2;
   t.chunk = smallest_chunk(precision, t.lanes_per_solve, n_layer);
@@ -724,7 +724,7 @@ TileConfig choose_tile(int precision, int mode, int n_layer, bool keqv, int nd_p
     }
   }
   if (!tuned) {
-    if (t.lanes_per_solve <= 0) t.lanes_per_solve = built_in_lanes(precision, mode, n_layer, keqv);
+    if (t.lanes_per_solve <= 0) t.lanes_per_solve = built_in_lanes(precision, n_layer, keqv);
     if (t.warps_per_cta <= 0) t.warps_per_cta = built_in_warps(precision, keqv, nd_profile);
     t.chunk = 0;
   }
@@ -1185,7 +1185,7 @@ int launch_flux(const FluxParams &p, const socgpu_control *c, cudaStream_t st, c
   const int mode = mode_index(c);
   TileConfig t = choose_tile(c->precision, mode, p.n_layer, p.keqv, p.nd_profile);
   // options the phased kernel does not cover run on the scan kernels
-  if (t.lanes_per_solve == 1 && !phased_supported(p)) t = scan_tile(c->precision, mode, p.n_layer, p.keqv, p.nd_profile);
+  if (t.lanes_per_solve == 1 && !phased_supported(p)) t = scan_tile(c->precision, p.n_layer, p.keqv, p.nd_profile);
   const FluxVariant *v = find_variant(c->precision, mode, t.lanes_per_solve);
   if (v && t.lanes_per_solve == 1) return v->launch(p, t, st, msg, msg_len);
   if (!v || t.chunk == 0) {
@@ -1656,7 +1656,7 @@ int build_plan(socgpu_batch_s &b, char *msg, size_t msg_len) {
   for (size_t i = 0; i < b.params.size(); ++i) {
     TileConfig t = choose_tile(b.precision[i], b.mode[i], b.params[i].n_layer, b.params[i].keqv, b.params[i].nd_profile);
     // the phased kernel has no persistent multi-batch form
-    if (t.lanes_per_solve == 1) t = scan_tile(b.precision[i], b.mode[i], b.params[i].n_layer, b.params[i].keqv, b.params[i].nd_profile);
+    if (t.lanes_per_solve == 1) t = scan_tile(b.precision[i], b.params[i].n_layer, b.params[i].keqv, b.params[i].nd_profile);
     classes[std::make_tuple(b.precision[i], b.mode[i], t.lanes_per_solve, t.chunk, t.warps_per_cta,
                             b.params[i].isolir, b.params[i].region)].push_back((int)i);
   }

@@ -44,6 +44,7 @@
 namespace socgpu {
 
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kTauBlock = 4;      // layers of a lane whose McICA cells are evaluated together
 
 // Bounds of a cell's absorption depth: from below the FP64 reference's cap
 // on the single-scattering albedo (1 - omega >= 32 epsilon) and a floor that
@@ -183,6 +184,12 @@ template <int P, int CH, bool NOSCAT, bool MCICA, int SRC, class Sm>
 struct TauSolve {
   static constexpr int LP = P * CH;
   static constexpr bool kLw = SRC == SOCGPU_IP_INFRA_RED;
+  // McICA cells are evaluated in a rolled loop, kBlock layers of the lane at a
+  // time, and handed to the unrolled elimination through shared memory (a
+  // lane reads back what it wrote): unrolled, the cell with its cloud types
+  // is more code than the instruction cache holds (solar, 8000 x 85 in the 8 x
+  // 11 tile: 7.1 of 16 stall cycles per instruction were fetches, 1450 us).
+  static constexpr int kBlock = MCICA ? kTauBlock : CH;
 
   // The band's staged optics and, in a cloudy solve, the subcolumn.
   struct Band {
@@ -192,6 +199,9 @@ struct TauSolve {
     const float *tkd;          // [LP] unscaled grey depth (i_direct_tau = ip_direct_noscaling), else null
     const float *fm1;          // [LP] adjust_solar_ke - 1 (k_eqv_scl, solar), else null
     const float *dB, *dB2;
+    const float *kg;           // [LP] the gas absorption where it is not k0 in every layer, else null
+    float k0;
+    __device__ __forceinline__ float gas(int s) const { return kg ? kg[s] : k0; }
   };
 
   // Cloud types present in slot s of a cloudy solve (at most two, bit t).
@@ -224,8 +234,9 @@ struct TauSolve {
   // lane evaluates one cell whether it is clear or holds one type, so the
   // lanes of a warp do not diverge.
   __device__ static __forceinline__ CellT cell(const FluxParams &p, const Sm &S, const SchemeT &sc, const Band &b,
-                                               int s, float kg, float sec0) {
+                                               int s, float sec0) {
     const float4 o = b.opt[s];
+    const float kg = b.gas(s);
     float a = fmaf(kg, o.w, o.x), sd = o.y, sg = o.z;
     if (!MCICA || !b.cs)
       return cell_tau<SRC, NOSCAT>(sc, p.l_ir_source_quad, bound_abs(a, sd), sd, sg, sec0);
@@ -247,10 +258,9 @@ struct TauSolve {
   // The direct transmission of slot s (UNSCALED: of the depth before
   // delta-rescaling), times the k_eqv_scl factor.
   template <bool UNSCALED>
-  __device__ static __forceinline__ float direct(const FluxParams &p, const Sm &S, const Band &b, int s, float kg,
-                                                 float sec0) {
+  __device__ static __forceinline__ float direct(const FluxParams &p, const Sm &S, const Band &b, int s, float sec0) {
     const float4 o = b.opt[s];
-    const float gas = kg * o.w, grey = UNSCALED ? b.tkd[s] : o.x + o.y, zk = -kLog2e * sec0;
+    const float gas = b.gas(s) * o.w, grey = UNSCALED ? b.tkd[s] : o.x + o.y, zk = -kLog2e * sec0;
     float T0;
     unsigned types = 0u;
     float cs = 0.0f;
@@ -269,14 +279,9 @@ struct TauSolve {
     }
     return b.fm1 ? fmaf(T0, b.fm1[s], T0) : T0;
   }
-  // The beam at the chunk top and at the surface, f_inc = 1: an exclusive
-  // product scan of the chunks' transmissions.
-  template <bool UNSCALED>
-  __device__ static __forceinline__ float beam(const FluxParams &p, const Sm &S, const Band &b, const float (&kg)[CH],
-                                               int r, float sec0, float &bottom) {
-    float incl = 1.0f;
-#pragma unroll
-    for (int j = 0; j < CH; ++j) incl *= direct<UNSCALED>(p, S, b, j * P + r, kg[j], sec0);
+  // The beam at the chunk top and at the surface for f_inc = 1, from the
+  // chunk's transmission: an exclusive product scan.
+  __device__ static __forceinline__ float beam_scan(float incl, int r, float &bottom) {
 #pragma unroll
     for (int d = 1; d < P; d <<= 1) {
       const float y = __shfl_up_sync(0xffffffffu, incl, d, P);
@@ -286,35 +291,51 @@ struct TauSolve {
     const float top = __shfl_up_sync(0xffffffffu, incl, 1, P);
     return r == 0 ? 1.0f : top;
   }
+  // The unscaled beam (ip_direct_noscaling, solar_source.F90:157-176): the
+  // reported direct flux; returns it at the surface.
+  __device__ static __forceinline__ float unscaled_beam(const FluxParams &p, const Sm &S, const Band &b, int r,
+                                                        float sec0, float f_inc, float w, float *accd) {
+    float t = 1.0f, bottom;
+#pragma unroll 1
+    for (int j = 0; j < CH; ++j) t *= direct<true>(p, S, b, j * P + r, sec0);
+    float f = f_inc * beam_scan(t, r, bottom);
+    if (r == 0) accd[LP] += w * f;
+#pragma unroll 1
+    for (int j = 0; j < CH; ++j) {
+      f *= direct<true>(p, S, b, j * P + r, sec0);
+      accd[j * P + r] += w * f;
+    }
+    return f_inc * bottom;
+  }
 
   // acc2: the group's (up, divergence) per slot, slot LP holding (up at the
   // top, down at the top); accd: its direct flux per slot (solar) or its
   // downward flux (without scattering).  w: the weight.
-  __device__ static __forceinline__ void solve(const FluxParams &p, const Sm &S, const Band &b, const float (&kg)[CH],
-                                               int r, float sec0, const float *bs, float w, float2 *acc2,
-                                               float *accd) {
+  // buf: the lane's kBlock cells (McICA), 32 lanes apart.
+  __device__ static __forceinline__ void solve(const FluxParams &p, const Sm &S, const Band &b, int r, float sec0,
+                                               const float *bs, float w, float2 *acc2, float *accd, float4 *buf) {
     const SchemeT sc(p);
     const float f_inc_down = bs[0], alb = bs[2];
     float fd = 0.0f, src = 0.0f;
-    if constexpr (!kLw) {
-      float bottom;
-      fd = bs[1] * beam<false>(p, S, b, kg, r, sec0, bottom);
-      if (b.tkd) {
-        // ip_direct_noscaling (solar_source.F90:157-176): the reported direct
-        // flux and the ground's direct reflection take the unscaled beam
-        float fu = bs[1] * beam<true>(p, S, b, kg, r, sec0, bottom);
-        if (r == 0) accd[LP] += w * fu;
+    // the beam runs relative to the chunk top under McICA (a pass over the
+    // cells for the chunk's transmission would evaluate their clouds twice);
+    // under clear skies that pass is cheaper than keeping the beam per layer
+    constexpr bool kRel = MCICA && !kLw;
+    if constexpr (!kLw && !kRel) {
+      float t = 1.0f, bottom;
 #pragma unroll
-        for (int j = 0; j < CH; ++j) {
-          fu *= direct<true>(p, S, b, j * P + r, kg[j], sec0);
-          accd[j * P + r] += w * fu;
-        }
-      } else if (r == 0) {
-        accd[LP] += w * fd;
+      for (int j = 0; j < CH; ++j) t *= direct<false>(p, S, b, j * P + r, sec0);
+      fd = bs[1] * beam_scan(t, r, bottom);
+      if (b.tkd) bottom = unscaled_beam(p, S, b, r, sec0, bs[1], w, accd);
+      else {
+        if (r == 0) accd[LP] += w * fd;
+        bottom *= bs[1];
       }
-      src = (bs[3] - alb) * bs[1] * bottom;
-    } else {
+      src = (bs[3] - alb) * bottom;
+    } else if constexpr (kLw) {
       src = (1.0f - alb) * bs[4];
+    } else {
+      fd = 1.0f;
     }
 
     if constexpr (NOSCAT) {
@@ -324,7 +345,7 @@ struct TauSolve {
 #pragma unroll
       for (int j = 0; j < CH; ++j) {
         const int s = j * P + r;
-        const CellT c = cell(p, S, sc, b, s, kg[j], sec0);
+        const CellT c = cell(p, S, sc, b, s, sec0);
         const float u = c.c1 * b.dB[s], q = p.l_ir_source_quad ? c.c2 * b.dB2[s] : 0.0f;
         T[j] = c.T; om[j] = c.om; su[j] = q + u; sd[j] = q - u;
         A = c.T * A; B = fmaf(c.T, B, sd[j]);
@@ -375,10 +396,28 @@ struct TauSolve {
     // j gives the layer's six coefficients, then takes the layer in
     float ca[CH], ce[CH], cg[CH], cp[CH], cq[CH], cv[CH];
     CompT c{0.0f, 0.0f, 1.0f, 0.0f, 0.0f};
+    float bt[kRel ? CH : 1];               // the beam below each layer, relative to the chunk top
 #pragma unroll
-    for (int j = 0; j < CH; ++j) {
+    for (int j0 = 0; j0 < CH; j0 += kBlock) {
+    if constexpr (MCICA) {
+#pragma unroll 1
+      for (int j = j0; j < min(j0 + kBlock, CH); ++j) {
+        const CellT x = cell(p, S, sc, b, j * P + r, sec0);
+        buf[(j - j0) * 32] = make_float4(x.T, x.R, x.T0, x.c1);
+        ((float2 *)(buf + kBlock * 32 - threadIdx.x % 32))[(j - j0) * 32 + threadIdx.x % 32] = make_float2(x.c2, x.om);
+      }
+    }
+#pragma unroll
+    for (int j = j0; j < (j0 + kBlock < CH ? j0 + kBlock : CH); ++j) {
       const int s = j * P + r;
-      const CellT x = cell(p, S, sc, b, s, kg[j], sec0);
+      CellT x;
+      if constexpr (MCICA) {
+        const float4 u = buf[(j - j0) * 32];
+        const float2 v = ((const float2 *)(buf + kBlock * 32 - threadIdx.x % 32))[(j - j0) * 32 + threadIdx.x % 32];
+        x = CellT{u.x, u.y, u.z, u.w, v.x, v.y};
+      } else {
+        x = cell(p, S, sc, b, s, sec0);
+      }
       float su, sd, ss;
       if constexpr (!kLw) {
         float T0 = x.T0, c2 = x.c2;
@@ -390,7 +429,8 @@ struct TauSolve {
         su = x.c1 * fd; sd = c2 * fd;        // solar_source.F90:146-155
         ss = su + sd;
         fd *= T0;
-        if (!b.tkd) accd[s] += w * fd;
+        if constexpr (kRel) bt[j] = fd;
+        else if (!b.tkd) accd[s] += w * fd;
       } else {                               // ir_source.F90:93-119
         const float u = x.c1 * b.dB[s], q = p.l_ir_source_quad ? x.c2 * b.dB2[s] : 0.0f;
         su = q + u; sd = q - u; ss = q + q;
@@ -407,6 +447,22 @@ struct TauSolve {
       c.Sd = fmaf(a, fmaf(c.R2, su, c.Sd), sd);
       c.R2 = fmaf(x.T * c.R2, a, x.R);
       c.T *= a;
+    }
+    }
+    if constexpr (kRel) {
+      // the sources in the beam's own units
+      float bottom;
+      fd = bs[1] * beam_scan(fd, r, bottom);
+      c.Su *= fd; c.Sd *= fd;
+      bottom *= bs[1];
+      if (b.tkd) {
+        bottom = unscaled_beam(p, S, b, r, sec0, bs[1], w, accd);
+      } else {
+        if (r == 0) accd[LP] += w * fd;
+#pragma unroll
+        for (int j = 0; j < CH; ++j) accd[j * P + r] += (w * fd) * bt[j];
+      }
+      src = (bs[3] - alb) * bottom;
     }
     // the stack above this chunk: an inclusive scan, shifted by one lane
     CompT pre = c;
@@ -447,9 +503,10 @@ struct TauSolve {
       const int s = j * P + r;
       float2 v = acc2[s];
       v.x = fmaf(w, fu, v.x);
-      v.y = fmaf(w, fmaf(cp[j], fu, fmaf(cq[j], fdt, cv[j])), v.y);
+      const float vj = kRel ? cv[j] * fd : cv[j], gj = kRel ? cg[j] * fd : cg[j];
+      v.y = fmaf(w, fmaf(cp[j], fu, fmaf(cq[j], fdt, vj)), v.y);
       acc2[s] = v;
-      fu = fmaf(ca[j], fu, fmaf(ce[j], fdt, cg[j]));
+      fu = fmaf(ca[j], fu, fmaf(ce[j], fdt, gj));
     }
     if (r == 0) { acc2[LP].x += w * fu; acc2[LP].y += w * f_inc_down; }
   }

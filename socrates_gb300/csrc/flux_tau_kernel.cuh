@@ -50,7 +50,8 @@ inline TauLayout tau_layout(const FluxParams &p, int LP, int P, int cols, int wa
   l.lki = p.lk_on ? take(n) : 0;
   l.sbf = p.n_sb > 0 ? take((size_t)p.n_sb * n) : 0;
   l.sbj = p.n_sb > 0 ? take((size_t)p.n_sb * n) : 0;
-  l.scr = p.term_scr ? take((size_t)n_groups * n) : 0;
+  // a group's row of gas absorption, where it is not one k for all layers
+  l.scr = (p.term_scr || p.max_abs > 1) ? take((size_t)n_groups * n) : 0;
   // a group's accumulators: the groups of a warp start P slots apart modulo
   // the 32 banks
   l.acc_stride = LP + 1;
@@ -68,9 +69,11 @@ inline TauLayout tau_layout(const FluxParams &p, int LP, int P, int cols, int wa
   return l;
 }
 
-// A CTA's shared memory: the columns' blocks and the band records.
+// A CTA's shared memory: the columns' blocks, the band records and under
+// McICA each warp's cells (six words for kTauBlock layers of every lane).
 inline size_t tau_bytes(const FluxParams &p) {
-  return (size_t)p.tau.stride * p.tau.cols + sizeof(BandLite) * p.tau.nbat;
+  const size_t cells = p.mcica ? (size_t)p.tau.cols * p.tau.warps * kTauBlock * 32 * 24 : 0;
+  return (size_t)p.tau.stride * p.tau.cols + sizeof(BandLite) * p.tau.nbat + cells;
 }
 
 // The columns per CTA, and the bands staged at a time, of a CTA of warps_cta
@@ -440,7 +443,7 @@ struct TauKernel {
   // One g-point: the clear solve and, under McICA, the solves of its
   // subcolumns with their blending weights (mcica_sample.F90:453-925).
   __device__ static __forceinline__ void gpoint(const FluxParams &p, const Sm &S, int col, int g, int bstart, float sec0,
-                                                int r, float2 *acc2, float *accd, bool active) {
+                                                int r, float2 *acc2, float *accd, float4 *buf, bool active) {
     const GPoint &gp = p.gpoints[g];
     const int b = gp.band, bi = b - bstart;
     const BandInfo &bd = p.bands[b];
@@ -456,16 +459,23 @@ struct TauKernel {
     bnd.fm1 = (!kLw && p.keqv) ? S.aux + row * p.max_abs : nullptr;
     bnd.dB = S.dB + row;
     bnd.dB2 = S.dB2 + row;
-    float kg[CH];
     if (single_gas(p, bd)) {
-      const float k0 = gp.kf[0];
-#pragma unroll
-      for (int j = 0; j < CH; ++j) kg[j] = k0;
+      bnd.kg = nullptr;
+      bnd.k0 = gp.kf[0];
+    } else if (!p.l_gas || gp.n_abs == 0) {
+      bnd.kg = nullptr;
+      bnd.k0 = 0.0f;
     } else {
+      // into the group's row (the lane's own slots)
+      float kg[CH];
       FK::gas_k_lane(p, S, FK::load_gas(gp, bd, p.max_abs), gp, bd, S.amt + row * p.max_abs, r, p.n_layer, kg);
+#pragma unroll
+      for (int j = 0; j < CH; ++j) S.scr[j * P + r] = kg[j];
+      bnd.kg = S.scr;
+      bnd.k0 = 0.0f;
     }
     if constexpr (!MCICA) {
-      Solve::solve(p, S, bnd, kg, r, sec0, bs, w_g, acc2, accd);
+      Solve::solve(p, S, bnd, r, sec0, bs, w_g, acc2, accd, nullptr);
     } else {
       const int iex = gp.iex_major;
       const int first = __ldg(p.first_subcol_k + b + (size_t)p.nd_band_sp * iex);
@@ -497,7 +507,7 @@ struct TauKernel {
           }
           bnd.cs = S.csub + (size_t)(j - 1) * LP;
         }
-        Solve::solve(p, S, bnd, kg, r, sec0, bs, w, acc2, accd);
+        Solve::solve(p, S, bnd, r, sec0, bs, w, acc2, accd, buf);
       }
     }
   }
@@ -516,20 +526,26 @@ struct TauKernel {
       const int c = q & (C - 1), lev = q / C;
       if (c >= nc) continue;
       unsigned char *b = base + (size_t)c * l.stride;
-      const float2 *acc2 = (const float2 *)(b + l.acc2);
+      float2 *acc2 = (float2 *)(b + l.acc2);
       const float *accd = (const float *)(b + l.accd);
       const int s = FK::level_slot(lev);
-      float u = 0.0f, d = 0.0f, dir = 0.0f;
+      // the rounding of the upward sum is kept: the downward flux is formed
+      // from it, and may be far smaller
+      float u = 0.0f, u_lo = 0.0f, d = 0.0f, dir = 0.0f;
       for (int k = 0; k < n_groups; ++k) {
         const float2 v = acc2[k * l.acc_stride + s];
-        u += v.x; d += v.y;
+        const float t = __fadd_rn(u, v.x), z = __fadd_rn(t, -u);
+        u_lo += __fadd_rn(__fadd_rn(u, -__fadd_rn(t, -z)), __fadd_rn(v.x, -z));
+        u = t;
+        d += v.y;
         if (kThird) dir += accd[k * l.accd_stride + s];
       }
+      if (!NOSCAT) acc2[s].x = u_lo;          // (this thread reads it back)
       float *up = up_of(c);
       up[lev] = u;
       // the top's second word is its downward flux, a layer's (at its bottom
       // level) the layer's divergence
-      if (lev == 0) { up[n1] = d - u; up[2 * n1 + L] = d; }
+      if (lev == 0) { up[n1] = (d - u) - u_lo; up[2 * n1 + L] = d; }
       else up[2 * n1 + lev - 1] = d;
       if (NOSCAT) up[n1 + lev] = dir;       // the downward flux in place of the net flux
       if (p.flux_direct) p.flux_direct[(size_t)(col0 + c) + ndp * lev] = kLw ? 0.0 : widen(dir);
@@ -567,8 +583,10 @@ struct TauKernel {
       const float *up = up_of(c);
       const size_t o = (size_t)(col0 + c) + ndp * lev;
       const float pl = kLw ? ((const float *)(b + l.pl))[FK::level_slot(lev)] : 0.0f, u = up[lev];
-      p.flux_up[o] = widen(u + pl);
-      p.flux_down[o] = widen(NOSCAT ? up[n1 + lev] + pl : lev == 0 ? up[2 * n1 + L] + pl : (up[n1 + lev] + u) + pl);
+      const float u_lo = NOSCAT ? 0.0f : ((const float2 *)(b + l.acc2))[FK::level_slot(lev)].x;
+      p.flux_up[o] = widen(u + (pl + u_lo));
+      p.flux_down[o] = widen(NOSCAT ? up[n1 + lev] + pl : lev == 0 ? up[2 * n1 + L] + pl
+                                                                   : ((up[n1 + lev] + u) + u_lo) + pl);
       if (lev < L) {
         const float d = up[2 * n1 + lev];
         if (p.flux_div) p.flux_div[o] = widen(d);
@@ -592,6 +610,8 @@ struct TauKernel {
     const int col = col0 + min(c, nc - 1);
     const float sec0 = (!kLw && p.zen_0) ? in_col(p.zen_0 + col) : 1.0f;
     BandLite *lite = (BandLite *)(smem + (size_t)C * l.stride);
+    // the warp's cells (McICA), this lane's
+    float4 *buf = (float4 *)(lite + l.nbat) + warp * (Solve::kBlock * 48) + lane;
     float2 *acc2 = S.acc2 + (size_t)gi * l.acc_stride;
     float *accd = S.accd + (size_t)gi * l.accd_stride;
     for (int q = wi * 32 + lane; q < n_groups * l.acc_stride; q += l.warps * 32) S.acc2[q] = make_float2(0.0f, 0.0f);
@@ -629,7 +649,7 @@ struct TauKernel {
         // full-warp shuffles see all lanes
         for (int g0 = g_lo + wi * gw; g0 < g_hi; g0 += n_groups) {
           const int g = g0 + lane / P;
-          gpoint(p, S, col, g < g_hi ? g : g_lo, bstart, sec0, r, acc2, accd, g < g_hi);
+          gpoint(p, S, col, g < g_hi ? g : g_lo, bstart, sec0, r, acc2, accd, buf, g < g_hi);
         }
         if (kLw) {
           // the band Planck fluxes of adjust_ir_radiance.F90:75-95

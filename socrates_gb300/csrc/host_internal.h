@@ -65,7 +65,7 @@ int mode_index(const socgpu_control *c);
 TileConfig choose_tile(int precision, int mode, int n_layer, bool keqv, int nd_profile);
 // The built-in tile of the scan kernels (flux_kernel), for launches the
 // phased kernel does not take (persistent multi-batch classes).
-TileConfig scan_tile(int precision, int mode, int n_layer, bool keqv, int nd_profile);
+TileConfig scan_tile(int precision, int n_layer, bool keqv, int nd_profile);
 
 using LaunchFn = int (*)(const FluxParams &, const TileConfig &, cudaStream_t, char *, size_t);
 using PrepareFn = int (*)(BatchGroup &, char *, size_t);
