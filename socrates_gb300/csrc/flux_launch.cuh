@@ -110,7 +110,7 @@ int prepare_tau(BatchGroup &g, char *msg, size_t len) {
     g.col_start[i + 1] = g.col_start[i] + (p.n_profile + p.tau.cols - 1) / p.tau.cols;
   }
   g.total = g.col_start[g.n_items];
-  if (bytes > 48 * 1024) {
+  if (bytes + fa.sharedSizeBytes > 48 * 1024) {   // the limit covers both kinds
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -253,7 +253,7 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
     p.band_batch = batch;
   }
   const size_t dyn = smem;
-  if (dyn > 48 * 1024) {
+  if (dyn + fa.sharedSizeBytes > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) {
       cudaGetLastError();
