@@ -24,10 +24,13 @@
 // (i % CH) * P + i / CH, so lane r's j-th layer is slot j*P + r and the P
 // lanes of a group touch P consecutive words (no bank conflicts).
 //
-// The mixed-precision instantiation (R = float) does all of its arithmetic
-// in FP32: FP64 inputs are narrowed once while staging (on the integer
-// pipe), table constants come from FP32 copies, and results are widened on
-// the way out.  On GB300 the FP64 pipe runs at 1/64 of FP32.
+// The FP32 instantiation (R = float, FP64 I/O) runs cloud regions only; clear
+// skies and McICA in mixed precision run on the kernels of
+// flux_tau_kernel.cuh, which take the lookup tables, the minor absorbers and
+// the aerosol and cloud optics from here.  FP64 inputs are narrowed while
+// staging on the integer pipe, table constants come from FP32 copies, and
+// results are widened on the way out: on GB300 the FP64 pipe runs at 1/64 of
+// FP32.
 //
 // McICA (mcica_sample.F90:453-925, mcica_column.F90:261-602): a group loops
 // over the subcolumns assigned to its g-point plus the clear solve and adds
