@@ -1862,7 +1862,7 @@ struct FluxKernel {
   __device__ static void solve_regions(const FluxParams &p, const Smem &S, int g_lo, int g_hi, int bstart, R sec0) {
     constexpr bool lw = (SRC == SOCGPU_IP_INFRA_RED);
     const int L = p.n_layer, st = p.region_rt, nct = S.nct[0], nt = blockDim.x;
-    R *X = (R *)((unsigned char *)p.region_scr + (size_t)blockIdx.x * region_cta_bytes<R>(p));
+    R *X = (R *)((unsigned char *)p.region_scr + (size_t)blockIdx.x * p.region_stride);
     double *Y = (double *)(X + (size_t)(p.triple ? kRegRows3 : kRegRows) * (L + 1) * st);
     // the serial threads: CTAs take the SM's schedulers in turn
     const int t0 = ((int)threadIdx.x + nt - (int)(blockIdx.x * 64u) % nt) % nt;

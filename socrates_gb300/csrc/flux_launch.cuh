@@ -178,7 +178,8 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   if (MCICA && p.region) {
     grid = std::min(grid, region_ctas(kern, threads, lay.bytes));
     q.region_rt = region_rt(p);
-    if (scratch_alloc(&q.region_scr, region_cta_bytes<R>(q) * grid, st) != cudaSuccess) {
+    q.region_stride = region_cta_bytes<R>(q);
+    if (scratch_alloc(&q.region_scr, q.region_stride * grid, st) != cudaSuccess) {
       cudaGetLastError();
       snprintf(msg, len, "no device memory for the cloud regions' rows");
       return SOCGPU_I_ABORT_CALCULATION;
@@ -280,6 +281,7 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
       g.items[i].region_rt = region_rt(g.items[i]);
       cta = std::max(cta, region_cta_bytes<R>(g.items[i]));
     }
+    for (int i = 0; i < g.n_items; ++i) g.items[i].region_stride = cta;
     g.scratch = cta * g.grid;
   }
   }

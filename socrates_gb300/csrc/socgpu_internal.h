@@ -266,9 +266,12 @@ struct FluxParams {
   int type_region[4];                // the region (2 stratiform, 3 convective) of each 0-based cloud type
   TauLayout tau;                     // the mixed kernels' shared memory (set by the launcher)
   // cloud regions: threads (g-points) that solve at a time, and the rows of
-  // the resident CTAs in global memory (set by the launcher)
+  // the resident CTAs in global memory, region_stride bytes to a CTA (set by
+  // the launcher; one stride for all items of a launch, whose CTAs work on
+  // items of different heights at a time)
   int region_rt;
   void *region_scr;
+  size_t region_stride;
 };
 
 // Launch configuration chosen by the tuner.
