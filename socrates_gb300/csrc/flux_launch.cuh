@@ -60,9 +60,8 @@ int launch_tau(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   const size_t bytes = tau_bytes(q);
   auto kern = tau_kernel<S::P, S::CH, NOSCAT, MCICA, SRC>;
   if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e = allow_shared((const void *)kern, bytes);
     if (e != cudaSuccess) {
-      cudaGetLastError();
       snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
       return SOCGPU_I_ERR_RANGE;
     }
@@ -110,16 +109,13 @@ int prepare_tau(BatchGroup &g, char *msg, size_t len) {
     g.col_start[i + 1] = g.col_start[i] + (p.n_profile + p.tau.cols - 1) / p.tau.cols;
   }
   g.total = g.col_start[g.n_items];
-  if (bytes + fa.sharedSizeBytes > 48 * 1024) {   // the limit covers both kinds
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
-      return SOCGPU_I_ERR_RANGE;
-    }
+  cudaError_t e = allow_shared((const void *)kern, bytes);
+  if (e != cudaSuccess) {
+    snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
+    return SOCGPU_I_ERR_RANGE;
   }
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, bytes);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, bytes);
   if (e != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     snprintf(msg, len, "no CTA of %d threads and %zu bytes fits an SM", warps * 32, bytes);
@@ -166,9 +162,8 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   q.band_batch = batch;
   auto kern = flux_kernel<R, MIX, S::P, S::CH, NOSCAT, MCICA, SRC>;
   if (lay.bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes);
+    cudaError_t e = allow_shared((const void *)kern, lay.bytes);
     if (e != cudaSuccess) {
-      cudaGetLastError();
       snprintf(msg, len, "shared memory request of %zu bytes refused: %s", lay.bytes, cudaGetErrorString(e));
       return SOCGPU_I_ERR_RANGE;
     }
@@ -254,16 +249,13 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
     p.band_batch = batch;
   }
   const size_t dyn = smem;
-  if (dyn + fa.sharedSizeBytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      snprintf(msg, len, "shared memory request of %zu bytes refused: %s", dyn, cudaGetErrorString(e));
-      return SOCGPU_I_ERR_RANGE;
-    }
+  cudaError_t e = allow_shared((const void *)kern, dyn);
+  if (e != cudaSuccess) {
+    snprintf(msg, len, "shared memory request of %zu bytes refused: %s", dyn, cudaGetErrorString(e));
+    return SOCGPU_I_ERR_RANGE;
   }
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, dyn);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, dyn);
   if (e != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     snprintf(msg, len, "no CTA of %d threads and %zu bytes fits an SM", warps * 32, dyn);

@@ -50,9 +50,8 @@ int launch_phased_lp(const FluxParams &p, const TileConfig &cfg, cudaStream_t st
   q.band_batch = batch;
   auto kern = flux_kernel_phased<R, MIX, NOSCAT, SRC, LPM>;
   if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e = allow_shared((const void *)kern, bytes);
     if (e != cudaSuccess) {
-      cudaGetLastError();
       snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
       return SOCGPU_I_ERR_RANGE;
     }
