@@ -89,17 +89,19 @@ inline size_t tau_bytes(const FluxParams &p) {
 // and 270 us for one, two and four columns of the GA9 short wave, however few
 // share its SM, so the count with the least waves times that is taken (2000 x
 // 70: 327, 305, 280 us; 2500 x 70: 402, 444, 531).
-// The rule looks at the leading extent, not at the number of columns of the
-// call, so that a window of a batch sums in the same order as the whole.
+// The rule looks at the columns of the caller's call: a few columns in wide
+// arrays are spread like any other few (27 x 137 solar in arrays of 2500
+// columns: 57.5 us by the leading extent, 22.6 by the columns), and the windows that a
+// host call is cut into sum in the order of the whole call.
 // False: one band of one column does not fit.
 constexpr int kTauResident = 2 * 152;
 inline bool tau_fit(FluxParams &p, int LP, int P, int warps_cta, bool mcica, size_t cap) {
   const int nb_all = p.last_band - p.first_band + 1;
   const size_t want = std::min(cap, (size_t)(227 * 1024) * warps_cta / 16);
   const int resident = kTauResident * 8 / warps_cta;
-  int most = warps_cta % 4 != 0 || p.nd_profile <= resident ? 1 : p.nd_profile <= 2 * resident ? 2 : 4;
+  int most = warps_cta % 4 != 0 || p.width <= resident ? 1 : p.width <= 2 * resident ? 2 : 4;
   if (p.keqv && most == 4) {
-    const auto waves = [&](int c) { return (double)((p.nd_profile + c * resident - 1) / (c * resident)); };
+    const auto waves = [&](int c) { return (double)((p.width + c * resident - 1) / (c * resident)); };
     const double t1 = waves(1), t2 = 1.72 * waves(2), t4 = 3.1 * waves(4);
     most = t4 <= t1 && t4 <= t2 ? 4 : t2 <= t1 ? 2 : 1;
   }

@@ -181,6 +181,7 @@ struct FluxParams {
   int l_continuum, l_mixing_ratio, i_water;   // i_water: 0-based species of water vapour
   // sizes
   int n_profile, n_layer, nd_profile, nd_layer, id_ct;  // id_ct 0-based first cloudy layer
+  int width;                        // columns of the caller's call, of which n_profile may be a window
   int g_begin, g_end;               // g-point range of the band range
   int max_abs;                      // most absorbers of any band in the range (>= 1)
   int band_batch;                   // bands staged in shared memory at a time (set by the launcher)
