@@ -708,24 +708,21 @@ int built_in_lanes(int precision, int n_layer, bool keqv) {
   return n_layer <= 104 ? 8 : n_layer <= 144 ? 16 : 32;
 }
 
-// Warps per CTA of the built-in tile: under equivalent extinction, whose
-// minor absorbers leave lanes idle, four (GA9 short wave 2000 x 70 329 us, 350
-// with 8) unless the columns are too few to fill the SMs.
-int built_in_warps(int precision, bool keqv, int width) {
-  return precision == SOCGPU_PRECISION_MIXED && keqv && width > 304 ? 4 : 8;
-}
+// Warps per CTA of the built-in tile: eight; zero leaves them to the launcher,
+// which weighs columns against warps under equivalent extinction (tau_choose).
+int built_in_warps(int precision, bool keqv) { return precision == SOCGPU_PRECISION_MIXED && keqv ? 0 : 8; }
 
 // The built-in scan tile, with the smallest chunk covering the column.
-TileConfig scan_tile(int precision, int n_layer, bool keqv, int width) {
+TileConfig scan_tile(int precision, int n_layer, bool keqv) {
   TileConfig t{};
   t.lanes_per_solve = built_in_lanes(precision, n_layer, keqv);
-  t.warps_per_cta = built_in_warps(precision, keqv, width);
+  t.warps_per_cta = built_in_warps(precision, keqv);
   while (t.lanes_per_solve < 32 && smallest_chunk(precision, t.lanes_per_solve, n_layer) == 0) t.lanes_per_solve *= 2;
   t.chunk = smallest_chunk(precision, t.lanes_per_solve, n_layer);
   return t;
 }
 
-TileConfig choose_tile(int precision, int mode, int n_layer, bool keqv, int width) {
+TileConfig choose_tile(int precision, int mode, int n_layer, bool keqv) {
   TileConfig t{};
   bool tuned = false;
   {
@@ -739,7 +736,7 @@ TileConfig choose_tile(int precision, int mode, int n_layer, bool keqv, int widt
   }
   if (!tuned) {
     if (t.lanes_per_solve <= 0) t.lanes_per_solve = built_in_lanes(precision, n_layer, keqv);
-    if (t.warps_per_cta <= 0) t.warps_per_cta = built_in_warps(precision, keqv, width);
+    if (t.warps_per_cta <= 0) t.warps_per_cta = built_in_warps(precision, keqv);
     t.chunk = 0;
   }
   // the phased kernel's chunk is its k-term batch (0: the launcher's default)
@@ -1197,9 +1194,9 @@ int launch(const FluxParams &p, const socgpu_control *c, cudaStream_t st, char *
 namespace {
 int launch_flux(const FluxParams &p, const socgpu_control *c, cudaStream_t st, char *msg, size_t msg_len) {
   const int mode = mode_index(c);
-  TileConfig t = choose_tile(c->precision, mode, p.n_layer, p.keqv, p.width);
+  TileConfig t = choose_tile(c->precision, mode, p.n_layer, p.keqv);
   // options the phased kernel does not cover run on the scan kernels
-  if (t.lanes_per_solve == 1 && !phased_supported(p)) t = scan_tile(c->precision, p.n_layer, p.keqv, p.width);
+  if (t.lanes_per_solve == 1 && !phased_supported(p)) t = scan_tile(c->precision, p.n_layer, p.keqv);
   const FluxVariant *v = find_variant(c->precision, mode, t.lanes_per_solve);
   if (v && t.lanes_per_solve == 1) return v->launch(p, t, st, msg, msg_len);
   if (!v || t.chunk == 0) {
@@ -1693,9 +1690,9 @@ struct Branches {
 int build_plan(socgpu_batch_s &b, char *msg, size_t msg_len) {
   std::map<std::tuple<int, int, int, int, int, int, int>, std::vector<int>> classes;
   for (size_t i = 0; i < b.params.size(); ++i) {
-    TileConfig t = choose_tile(b.precision[i], b.mode[i], b.params[i].n_layer, b.params[i].keqv, b.params[i].width);
+    TileConfig t = choose_tile(b.precision[i], b.mode[i], b.params[i].n_layer, b.params[i].keqv);
     // the phased kernel has no persistent multi-batch form
-    if (t.lanes_per_solve == 1) t = scan_tile(b.precision[i], b.params[i].n_layer, b.params[i].keqv, b.params[i].width);
+    if (t.lanes_per_solve == 1) t = scan_tile(b.precision[i], b.params[i].n_layer, b.params[i].keqv);
     classes[std::make_tuple(b.precision[i], b.mode[i], t.lanes_per_solve, t.chunk, t.warps_per_cta,
                             b.params[i].isolir, b.params[i].region)].push_back((int)i);
   }

@@ -18,12 +18,31 @@ constexpr bool tau_form(const FluxParams &p) { return sizeof(R) == 4 && !(MCICA 
 
 constexpr int kRegionCtasPerSm = 4, kRegionWarps = 4;
 
-// Shared memory the current device grants one CTA.
-inline int smem_limit() {
-  int v = 0, dev = 0;
+inline TauChip tau_chip() {
+  int dev = 0, n = 0, cta = 0, sm = 0, kept = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return v;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  cudaDeviceGetAttribute(&kept, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+  return TauChip{n, (size_t)cta, (size_t)sm, (size_t)kept};
+}
+
+// The kernel of shape S built for mb resident CTAs (tau_min_ctas of them where
+// no other is built).
+template <bool NOSCAT, bool MCICA, int SRC, class S>
+auto tau_single(int mb) {
+  constexpr int least = tau_min_ctas(S::CH), most = tau_dense_ctas(S::P, S::CH, MCICA);
+  if constexpr (most >= 4) if (mb == 4) return tau_kernel<S::P, S::CH, NOSCAT, MCICA, SRC, 4>;
+  if constexpr (most >= 3) if (mb == 3) return tau_kernel<S::P, S::CH, NOSCAT, MCICA, SRC, 3>;
+  return tau_kernel<S::P, S::CH, NOSCAT, MCICA, SRC, least>;
+}
+template <bool NOSCAT, bool MCICA, int SRC, class S>
+auto tau_batched(int mb) {
+  constexpr int least = tau_min_ctas(S::CH), most = tau_dense_ctas(S::P, S::CH, MCICA);
+  if constexpr (most >= 4) if (mb == 4) return tau_kernel_batched<S::P, S::CH, NOSCAT, MCICA, SRC, 4>;
+  if constexpr (most >= 3) if (mb == 3) return tau_kernel_batched<S::P, S::CH, NOSCAT, MCICA, SRC, 3>;
+  return tau_kernel_batched<S::P, S::CH, NOSCAT, MCICA, SRC, least>;
 }
 
 // Threads that solve a cloud-region column's g-points at a time: whole warps
@@ -48,17 +67,25 @@ int region_ctas(K kern, int threads, size_t bytes) {
 template <bool NOSCAT, bool MCICA, int SRC, class S>
 int launch_tau(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char *msg, size_t len) {
   FluxParams q = p;
-  int warps = cfg.warps_per_cta;
-  const size_t cap = (size_t)smem_limit();
-  while (!tau_fit(q, S::P * S::CH, S::P, warps, MCICA, cap)) {
-    if (warps == 1) {
-      snprintf(msg, len, "one band of %d layers needs %u bytes of shared memory (limit %zu)", p.n_layer, q.tau.stride, cap);
-      return SOCGPU_I_ERR_RANGE;
+  int warps = cfg.warps_per_cta, mb = 0;
+  const TauChip chip = tau_chip();
+  const TauShape shape = tau_choose(&q, 1, S::P * S::CH, S::P, warps, MCICA, tau_dense_ctas(S::P, S::CH, MCICA), chip);
+  if (shape.warps) {
+    warps = shape.warps;
+    mb = shape.mb;
+  } else {
+    if (warps == 0) warps = 8;
+    while (!tau_fit(q, S::P * S::CH, S::P, warps, MCICA, chip)) {
+      if (warps == 1) {
+        snprintf(msg, len, "one band of %d layers needs %u bytes of shared memory (limit %zu)", p.n_layer, q.tau.stride,
+                 chip.cta);
+        return SOCGPU_I_ERR_RANGE;
+      }
+      warps /= 2;
     }
-    warps /= 2;
   }
   const size_t bytes = tau_bytes(q);
-  auto kern = tau_kernel<S::P, S::CH, NOSCAT, MCICA, SRC>;
+  auto kern = tau_single<NOSCAT, MCICA, SRC, S>(mb);
   if (bytes > 48 * 1024) {
     cudaError_t e = allow_shared((const void *)kern, bytes);
     if (e != cudaSuccess) {
@@ -81,28 +108,40 @@ int launch_tau(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
 // work in column groups, and a persistent grid.
 template <bool NOSCAT, bool MCICA, int SRC, class S>
 int prepare_tau(BatchGroup &g, char *msg, size_t len) {
-  int dev = 0, n_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-  const int warps = g.tile.warps_per_cta;
-  auto kern = tau_kernel_batched<S::P, S::CH, NOSCAT, MCICA, SRC>;
-  cudaFuncAttributes fa{};
-  if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) {
+  for (int i = 0; i < g.n_items; ++i)
+    if (g.items[i].n_layer > S::P * S::CH) {
+      snprintf(msg, len, "batch %d has %d layers, more than the %d of its tile", i, g.items[i].n_layer, S::P * S::CH);
+      return SOCGPU_I_ERR_RANGE;
+    }
+  TauChip chip = tau_chip();
+  const size_t optin = chip.cta;
+  // the kernel's static shared memory (its parameter copy) counts too
+  auto static_of = [&](const void *kern) {
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, kern) == cudaSuccess) return (long long)fa.sharedSizeBytes;
     cudaGetLastError();
     snprintf(msg, len, "attributes of the batched kernel not available");
-    return SOCGPU_I_ABORT_CALCULATION;
+    return -1LL;
+  };
+  auto kern = tau_batched<NOSCAT, MCICA, SRC, S>(0);
+  const long long fixed = static_of((const void *)kern);
+  if (fixed < 0) return SOCGPU_I_ABORT_CALCULATION;
+  chip.cta = optin - std::min(optin, (size_t)fixed);
+  chip.besides += (size_t)fixed;
+  int warps = g.tile.warps_per_cta;
+  const TauShape shape = tau_choose(g.items, g.n_items, S::P * S::CH, S::P, warps, MCICA,
+                                    tau_dense_ctas(S::P, S::CH, MCICA), chip);
+  if (shape.warps) {
+    warps = shape.warps;
+    kern = tau_batched<NOSCAT, MCICA, SRC, S>(shape.mb);
+  } else if (warps == 0) {
+    warps = 8;
   }
-  // the kernel's static shared memory (its parameter copy) counts too
-  const size_t cap = (size_t)smem_limit() - std::min((size_t)smem_limit(), fa.sharedSizeBytes);
   size_t bytes = 0;
   for (int i = 0; i < g.n_items; ++i) {
     FluxParams &p = g.items[i];
-    if (p.n_layer > S::P * S::CH) {
-      snprintf(msg, len, "batch %d has %d layers, more than the %d of its tile", i, p.n_layer, S::P * S::CH);
-      return SOCGPU_I_ERR_RANGE;
-    }
-    if (!tau_fit(p, S::P * S::CH, S::P, warps, MCICA, cap)) {
-      snprintf(msg, len, "batch %d: one band needs %u bytes of shared memory (limit %zu)", i, p.tau.stride, cap);
+    if (!shape.warps && !tau_fit(p, S::P * S::CH, S::P, warps, MCICA, chip)) {
+      snprintf(msg, len, "batch %d: one band needs %u bytes of shared memory (limit %zu)", i, p.tau.stride, chip.cta);
       return SOCGPU_I_ERR_RANGE;
     }
     bytes = std::max(bytes, tau_bytes(p));
@@ -124,7 +163,7 @@ int prepare_tau(BatchGroup &g, char *msg, size_t len) {
   g.kernel = (const void *)kern;
   g.smem = bytes;
   g.threads = warps * 32;
-  g.grid = (int)std::min<long long>(g.total, (long long)per_sm * n_sm);
+  g.grid = (int)std::min<long long>(g.total, (long long)per_sm * chip.n_sm);
   return 0;
 }
 
@@ -145,7 +184,9 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   // widest band batch (then most warps) whose staging fits in shared memory
-  int warps = MCICA && p.region ? std::min(cfg.warps_per_cta, kRegionWarps) : cfg.warps_per_cta, batch = nb;
+  // (no warps are given for mixed equivalent extinction: cloud regions here)
+  const int given = cfg.warps_per_cta > 0 ? cfg.warps_per_cta : 8;
+  int warps = MCICA && p.region ? std::min(given, kRegionWarps) : given, batch = nb;
   SmemLayout lay{};
   for (;;) {
     lay = make_layout<R>(p, S::P * S::CH, S::P, batch, warps * 32 / S::P, MCICA,
@@ -209,7 +250,8 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
   const bool region = MCICA && g.n_items > 0 && g.items[0].region;
-  const int warps = region ? std::min(g.tile.warps_per_cta, kRegionWarps) : g.tile.warps_per_cta;
+  const int given = g.tile.warps_per_cta > 0 ? g.tile.warps_per_cta : 8;
+  const int warps = region ? std::min(given, kRegionWarps) : given;
   const int n_groups = warps * 32 / S::P;
   auto bytes_of = [&](const FluxParams &p, int batch) {
     return make_layout<R>(p, S::P * S::CH, S::P, batch, n_groups, MCICA,
@@ -338,8 +380,10 @@ int preload_chunks() {
      ...);
   }
   if constexpr (sizeof(R) == 4) {
-    ((ok = ok && cudaFuncGetAttributes(&a, tau_kernel<P, CH, NOSCAT, MCICA, SRC>) == cudaSuccess), ...);
-    ((ok = ok && cudaFuncGetAttributes(&a, tau_kernel_batched<P, CH, NOSCAT, MCICA, SRC>) == cudaSuccess), ...);
+    for (int mb = 0; mb <= 4; ++mb) {
+      ((ok = ok && cudaFuncGetAttributes(&a, tau_single<NOSCAT, MCICA, SRC, Shape<P, CH>>(mb)) == cudaSuccess), ...);
+      ((ok = ok && cudaFuncGetAttributes(&a, tau_batched<NOSCAT, MCICA, SRC, Shape<P, CH>>(mb)) == cudaSuccess), ...);
+    }
   }
   if (!ok) cudaGetLastError();
   return ok ? 0 : SOCGPU_I_ABORT_CALCULATION;

@@ -76,44 +76,90 @@ inline size_t tau_bytes(const FluxParams &p) {
   return (size_t)p.tau.stride * p.tau.cols + sizeof(BandLite) * p.tau.nbat + cells;
 }
 
-// The columns per CTA, and the bands staged at a time, of a CTA of warps_cta
+// What the current device grants a kernel: SMs, dynamic shared memory of a CTA,
+// shared memory of an SM, and what a resident CTA takes of it besides (the
+// device's 1 KB and the kernel's static part).
+struct TauChip { int n_sm; size_t cta, sm, besides; };
+
+// The layout of batch p with `cols` columns to a CTA of `warps` warps: the most
+// bands at a time, at least `least`, that leave 16 warps resident; one band of
+// one column may take all of a CTA's shared memory.
+inline bool tau_place(FluxParams &p, int LP, int P, int warps, int cols, int least, bool mcica, const TauChip &chip) {
+  const size_t want = std::min(chip.cta, chip.cta * warps / 16);
+  for (int nb = p.last_band - p.first_band + 1; nb >= least; --nb) {
+    p.tau = tau_layout(p, LP, P, cols, warps / cols, nb, mcica);
+    const size_t bytes = tau_bytes(p);
+    if (bytes <= want || (nb == 1 && cols == 1 && bytes <= chip.cta)) return true;
+  }
+  return false;
+}
+
+// The columns per CTA, and the bands staged at a time, of a CTA of `warps`
 // warps.  Few columns are spread over the SMs, one or two to a CTA while the
-// chip holds them all at a time (kTauResident CTAs of 8 warps); past that,
+// chip holds them all at a time (16 warps to an SM); past that,
 // four adjacent columns if all their bands fit the share of shared memory
 // that leaves 16 warps resident, else two with at least half the bands; else
 // one.  Measured on GB300 (us, mixed, 8 warps): solar 10000 x 100 454 with
 // four columns, 475 with two, 715 with one; long wave 1000 x 60 39, 52, 78;
 // scattering long wave 3001 x 137 377 (bands in batches), 364, 393; solar
-// McICA 8000 x 85 1400 (in batches), 1252, 1445.  Under equivalent
-// extinction the minor absorbers dominate: a CTA of 4 warps takes 87, 150
-// and 270 us for one, two and four columns of the GA9 short wave, however few
-// share its SM, so the count with the least waves times that is taken (2000 x
-// 70: 327, 305, 280 us; 2500 x 70: 402, 444, 531).
+// McICA 8000 x 85 1400 (in batches), 1252, 1445.
 // The rule looks at the columns of the caller's call: a few columns in wide
 // arrays are spread like any other few (27 x 137 solar in arrays of 2500
 // columns: 57.5 us by the leading extent, 22.6 by the columns), and the windows that a
 // host call is cut into sum in the order of the whole call.
 // False: one band of one column does not fit.
-constexpr int kTauResident = 2 * 152;
-inline bool tau_fit(FluxParams &p, int LP, int P, int warps_cta, bool mcica, size_t cap) {
-  const int nb_all = p.last_band - p.first_band + 1;
-  const size_t want = std::min(cap, (size_t)(227 * 1024) * warps_cta / 16);
-  const int resident = kTauResident * 8 / warps_cta;
-  int most = warps_cta % 4 != 0 || p.width <= resident ? 1 : p.width <= 2 * resident ? 2 : 4;
-  if (p.keqv && most == 4) {
-    const auto waves = [&](int c) { return (double)((p.width + c * resident - 1) / (c * resident)); };
-    const double t1 = waves(1), t2 = 1.72 * waves(2), t4 = 3.1 * waves(4);
-    most = t4 <= t1 && t4 <= t2 ? 4 : t2 <= t1 ? 2 : 1;
-  }
-  for (int cols = most; cols >= 1; cols /= 2) {
-    const int least = cols == 4 ? (p.keqv ? 1 : nb_all) : cols == 2 ? (nb_all + 1) / 2 : 1;
-    for (int nb = nb_all; nb >= least; --nb) {
-      p.tau = tau_layout(p, LP, P, cols, warps_cta / cols, nb, mcica);
-      const size_t bytes = tau_bytes(p);
-      if (bytes <= want || (nb == 1 && cols == 1 && bytes <= cap)) return true;
-    }
-  }
+inline bool tau_fit(FluxParams &p, int LP, int P, int warps, bool mcica, const TauChip &chip) {
+  const int resident = 16 * chip.n_sm / warps, nb = p.last_band - p.first_band + 1;
+  const int most = warps % 4 != 0 || p.width <= resident ? 1 : p.width <= 2 * resident ? 2 : 4;
+  for (int cols = most; cols >= 1; cols /= 2)
+    if (tau_place(p, LP, P, warps, cols, cols == 4 ? nb : cols == 2 ? (nb + 1) / 2 : 1, mcica, chip)) return true;
   return false;
+}
+
+// Equivalent extinction, whose minor absorbers' solves leave most of a CTA
+// waiting: the time of one wave of CTAs grows little with the columns on an
+// SM, and with the columns a warp takes one after another.  The shape with the
+// least (waves x time of a wave) is taken, each at the residence that its
+// registers and shared memory allow.  The relative times are those of the GA9
+// short wave and long wave over 38 to 137 layers and 300 to 4000 columns on
+// GB300, which agree to a fifth (us for a full wave, short wave at 38 / 70 / 137
+// layers: one column on 8 warps 50 / 60 / 71, at three CTAs to an SM 54 / 67,
+// one on 4 warps 71 / 87 / 144, two 111 / 157 / 240, four 193 / 283 / 350).  With
+// one line between 8 and 4 warps at 304 columns and never more than 16 resident
+// warps it was slower than this by up to a third (38 x 400 69 us, now 54;
+// long wave 38 x 700 173, now 121).
+struct TauShape { int warps, cols, mb; double time; };   // mb: resident CTAs of 8 warps in registers
+constexpr TauShape kKeqvShapes[] = {{8, 1, 2, 1.0}, {8, 1, 3, 1.1}, {8, 1, 4, 1.35}, {4, 1, 2, 1.5},
+                                    {4, 1, 3, 1.6}, {4, 2, 2, 2.6}, {4, 4, 2, 4.65}};
+// The shape of n items that run together (of `given` warps unless that is 0) on
+// a tile built for up to `dense` resident CTAs, and the items' layouts; warps
+// 0: none fits, or an item is not of equivalent extinction.
+inline TauShape tau_choose(FluxParams *items, int n, int LP, int P, int given, bool mcica, int dense, const TauChip &chip) {
+  TauShape best{0, 0, 0, 0.0};
+  double least = 0.0;
+  for (int i = 0; i < n; ++i)
+    if (!items[i].keqv) return best;
+  for (const TauShape &s : kKeqvShapes) {
+    if (s.mb > std::max(dense, 2) || (given && s.warps != given)) continue;
+    size_t bytes = 0;
+    long long ctas = 0;
+    bool fits = true;
+    for (int i = 0; i < n && fits; ++i) {
+      const int nb = items[i].last_band - items[i].first_band + 1;
+      fits = tau_place(items[i], LP, P, s.warps, s.cols, s.cols == 2 ? (nb + 1) / 2 : 1, mcica, chip);
+      bytes = std::max(bytes, tau_bytes(items[i]));
+      ctas += (items[i].width + s.cols - 1) / s.cols;
+    }
+    if (!fits) continue;
+    const long long on_sm = std::max<long long>(1, std::min<long long>(std::min(s.mb, dense) * 8 / s.warps, chip.sm / (bytes + chip.besides)));
+    const double t = s.time * (double)((ctas + on_sm * chip.n_sm - 1) / (on_sm * chip.n_sm));
+    if (best.warps == 0 || t < least) { best = s; least = t; }
+  }
+  for (int i = 0; i < n && best.warps; ++i) {
+    const int nb = items[i].last_band - items[i].first_band + 1;
+    tau_place(items[i], LP, P, best.warps, best.cols, best.cols == 2 ? (nb + 1) / 2 : 1, mcica, chip);
+  }
+  return best;
 }
 
 // A value of the caller's column arrays.  The staging reads each once, so it
@@ -670,21 +716,29 @@ struct TauKernel {
   }
 };
 
-// Resident warps asked of the register allocator: 16 per SM (128 registers)
-// for chunks up to 13 layers, 8 above.  More for the short chunks did not
-// pay: at 24 and 32 resident warps (80 and 64 registers) solar McICA 8000 x
-// 85 takes 1399 and 1373 us instead of 1253.
+// Resident CTAs of 8 warps asked of the register allocator: 16 warps per SM (128
+// registers) for chunks up to 13 layers, 8 above.  More for the short chunks
+// did not pay under McICA: at 24 and 32 resident warps (80 and 64 registers)
+// solar McICA 8000 x 85 takes 1399 and 1373 us instead of 1253.
 constexpr int tau_min_ctas(int ch) { return ch <= 13 ? 2 : 1; }
+// The most that a shape is built for beside that, for columns that have a CTA
+// to themselves (tau_choose): the built-in tiles of equivalent extinction with
+// short chunks, whose solves wait more than they issue.  With four and five
+// layers on 32 lanes it did not pay (GA9 short wave 100 x 304 62 us at two CTAs,
+// 64 at three; 137 x 608 143 and 150).
+constexpr int tau_dense_ctas(int P, int ch, bool mcica) {
+  return mcica ? tau_min_ctas(ch) : P == 16 && ch == 3 ? 4 : (P == 16 && ch == 4) || (P == 32 && ch == 3) ? 3 : tau_min_ctas(ch);
+}
 
-template <int P, int CH, bool NOSCAT, bool MCICA, int SRC>
-__global__ void __launch_bounds__(256, tau_min_ctas(CH)) tau_kernel(const __grid_constant__ FluxParams p) {
+template <int P, int CH, bool NOSCAT, bool MCICA, int SRC, int MB>
+__global__ void __launch_bounds__(256, MB) tau_kernel(const __grid_constant__ FluxParams p) {
   TauKernel<P, CH, NOSCAT, MCICA, SRC>::run(p, blockIdx.x);
 }
 
 // Persistent form over many batches (flux_kernel_batched): the work indices
 // count groups of tau.cols columns.
-template <int P, int CH, bool NOSCAT, bool MCICA, int SRC>
-__global__ void __launch_bounds__(256, tau_min_ctas(CH))
+template <int P, int CH, bool NOSCAT, bool MCICA, int SRC, int MB>
+__global__ void __launch_bounds__(256, MB)
 tau_kernel_batched(const FluxParams *__restrict__ items, const long long *__restrict__ col_start, int n_items,
                    long long total) {
   __shared__ __align__(16) FluxParams sp;

@@ -251,8 +251,8 @@ void launch_wave(socgpu_server_s &S, StreamSlot &sl) {
     Request *r = wave[i];
     r->call.params(S.dmem + r->off, params[i]);
     const int mode = mode_index(&r->control);
-    TileConfig t = choose_tile(r->control.precision, mode, r->atm.n_layer, params[i].keqv, params[i].width);
-    if (t.lanes_per_solve == 1) t = scan_tile(r->control.precision, r->atm.n_layer, params[i].keqv, params[i].width);
+    TileConfig t = choose_tile(r->control.precision, mode, r->atm.n_layer, params[i].keqv);
+    if (t.lanes_per_solve == 1) t = scan_tile(r->control.precision, r->atm.n_layer, params[i].keqv);
     classes[std::make_tuple(r->control.precision, mode, t.lanes_per_solve, t.chunk, t.warps_per_cta,
                             r->control.isolir, params[i].region)].push_back((int)i);
   }

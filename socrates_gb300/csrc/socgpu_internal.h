@@ -278,7 +278,7 @@ struct FluxParams {
 // Launch configuration chosen by the tuner.
 struct TileConfig {
   int lanes_per_solve;   // P: lanes sharing one (column, g-point) solve
-  int warps_per_cta;     // warps per CTA; one CTA per column
+  int warps_per_cta;     // warps per CTA; 0 = the launcher's choice
   int chunk;             // CH: layers per lane; 0 = the smallest instantiated chunk that covers the column
 };
 
