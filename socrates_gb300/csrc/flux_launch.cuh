@@ -138,6 +138,7 @@ int prepare_tau(BatchGroup &g, char *msg, size_t len) {
     warps = 8;
   }
   size_t bytes = 0;
+  long long alone = 0;                  // CTAs with one column
   for (int i = 0; i < g.n_items; ++i) {
     FluxParams &p = g.items[i];
     if (!shape.warps && !tau_fit(p, S::P * S::CH, S::P, warps, MCICA, chip)) {
@@ -146,8 +147,11 @@ int prepare_tau(BatchGroup &g, char *msg, size_t len) {
     }
     bytes = std::max(bytes, tau_bytes(p));
     g.col_start[i + 1] = g.col_start[i] + (p.n_profile + p.tau.cols - 1) / p.tau.cols;
+    if (p.tau.cols == 1) alone += p.n_profile;
   }
   g.total = g.col_start[g.n_items];
+  if (!shape.warps && warps == 8 && 2 * alone > g.total && tau_narrow(g.total, chip))
+    kern = tau_batched<NOSCAT, MCICA, SRC, S>(3);
   cudaError_t e = allow_shared((const void *)kern, bytes);
   if (e != cudaSuccess) {
     snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));

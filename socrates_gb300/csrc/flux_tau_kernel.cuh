@@ -162,6 +162,17 @@ inline TauShape tau_choose(FluxParams *items, int n, int LP, int P, int given, b
   return best;
 }
 
+// Whether a class of ctas CTAs, most of them with one column on 8 warps, runs
+// with three of them resident on an SM in place of two: fewer waves, each a
+// tenth longer.  Graphs of 38-layer solar columns on GB300 (us): 32 items of
+// 16 columns 33 with two resident, 35 with three; 32 of 64 105 and 86; 16 of
+// 200 160 and 133; long wave without scattering 41 and 43, 131 and 105, 201
+// and 162.
+inline bool tau_narrow(long long ctas, const TauChip &chip) {
+  const auto waves = [&](long long n) { return (double)((ctas + n * chip.n_sm - 1) / (n * chip.n_sm)); };
+  return 1.1 * waves(3) < waves(2);
+}
+
 // A value of the caller's column arrays.  The staging reads each once, so it
 // does not take a line of the L1 cache, which holds the band tables.
 __device__ __forceinline__ double ld_col(const double *a) {
@@ -722,12 +733,13 @@ struct TauKernel {
 // solar McICA 8000 x 85 takes 1399 and 1373 us instead of 1253.
 constexpr int tau_min_ctas(int ch) { return ch <= 13 ? 2 : 1; }
 // The most that a shape is built for beside that, for columns that have a CTA
-// to themselves (tau_choose): the built-in tiles of equivalent extinction with
-// short chunks, whose solves wait more than they issue.  With four and five
+// to themselves (tau_choose, tau_narrow): the built-in tiles with short
+// chunks, whose few layers leave most of a CTA waiting.  With four and five
 // layers on 32 lanes it did not pay (GA9 short wave 100 x 304 62 us at two CTAs,
 // 64 at three; 137 x 608 143 and 150).
 constexpr int tau_dense_ctas(int P, int ch, bool mcica) {
-  return mcica ? tau_min_ctas(ch) : P == 16 && ch == 3 ? 4 : (P == 16 && ch == 4) || (P == 32 && ch == 3) ? 3 : tau_min_ctas(ch);
+  if (mcica) return tau_min_ctas(ch);
+  return P == 16 && ch == 3 ? 4 : (P == 16 && ch == 4) || (P == 32 && ch == 3) || (P == 8 && ch == 5) ? 3 : tau_min_ctas(ch);
 }
 
 template <int P, int CH, bool NOSCAT, bool MCICA, int SRC, int MB>
