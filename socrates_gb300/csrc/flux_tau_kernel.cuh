@@ -121,21 +121,24 @@ inline bool tau_fit(FluxParams &p, int LP, int P, int warps, bool mcica, const T
 // SM, and with the columns a warp takes one after another.  The shape with the
 // least (waves x time of a wave) is taken, each at the residence that its
 // registers and shared memory allow.  The relative times are those of the GA9
-// short wave and long wave over 38 to 137 layers and 300 to 4000 columns on
-// GB300, which agree to a fifth (us for a full wave, short wave at 38 / 70 / 137
-// layers: one column on 8 warps 50 / 60 / 71, at three CTAs to an SM 54 / 67,
-// one on 4 warps 71 / 87 / 144, two 111 / 157 / 240, four 193 / 283 / 350).  With
-// one line between 8 and 4 warps at 304 columns and never more than 16 resident
-// warps it was slower than this by up to a third (38 x 400 69 us, now 54;
-// long wave 38 x 700 173, now 121).
-struct TauShape { int warps, cols, mb; double time; };   // mb: resident CTAs of 8 warps in registers
-constexpr TauShape kKeqvShapes[] = {{8, 1, 2, 1.0}, {8, 1, 3, 1.1}, {8, 1, 4, 1.35}, {4, 1, 2, 1.5},
-                                    {4, 1, 3, 1.6}, {4, 2, 2, 2.6}, {4, 4, 2, 4.65}};
+// short-wave and long-wave files over 38 to 137 layers and 300 to 4000 columns
+// on GB300, which agree to a fifth (us of a full wave, short wave at 38 / 70 /
+// 137 layers: one column on 8 warps 50 / 60 / 71, at three CTAs to an SM 54 / 67,
+// one on 4 warps 71 / 87 / 144, two 111 / 157 / 240, four 193 / 283 / 350; under
+// McICA one on 4 warps takes 1.4 to 2.3 times one on 8, more with more layers
+// to a lane).  A line between 8 and 4 warps at 304 columns, with never more than
+// 16 resident warps, was slower than this by up to a third (38 x 400 69 us, now
+// 54; long wave 38 x 700 173, now 121).
+// mb: resident CTAs of 8 warps in registers; the relative times on tiles built
+// for three or more of them (short chunks) and on the others.
+struct TauShape { int warps, cols, mb; double time, time_long; };
+constexpr TauShape kKeqvShapes[] = {{8, 1, 2, 1.0, 1.0}, {8, 1, 3, 1.1, 0.0}, {8, 1, 4, 1.35, 0.0}, {4, 1, 2, 1.5, 1.9},
+                                    {4, 1, 3, 1.6, 0.0}, {4, 2, 2, 2.6, 3.1}, {4, 4, 2, 4.65, 5.0}};
 // The shape of n items that run together (of `given` warps unless that is 0) on
 // a tile built for up to `dense` resident CTAs, and the items' layouts; warps
 // 0: none fits, or an item is not of equivalent extinction.
 inline TauShape tau_choose(FluxParams *items, int n, int LP, int P, int given, bool mcica, int dense, const TauChip &chip) {
-  TauShape best{0, 0, 0, 0.0};
+  TauShape best{};
   double least = 0.0;
   for (int i = 0; i < n; ++i)
     if (!items[i].keqv) return best;
@@ -152,7 +155,9 @@ inline TauShape tau_choose(FluxParams *items, int n, int LP, int P, int given, b
     }
     if (!fits) continue;
     const long long on_sm = std::max<long long>(1, std::min<long long>(std::min(s.mb, dense) * 8 / s.warps, chip.sm / (bytes + chip.besides)));
-    const double t = s.time * (double)((ctas + on_sm * chip.n_sm - 1) / (on_sm * chip.n_sm));
+    double wave = dense > 2 ? s.time : s.time_long;
+    if (mcica && s.warps == 4 && s.cols == 1) wave = LP / P <= 3 ? 1.49 : LP / P == 4 ? 1.6 : 2.1;
+    const double t = wave * (double)((ctas + on_sm * chip.n_sm - 1) / (on_sm * chip.n_sm));
     if (best.warps == 0 || t < least) { best = s; least = t; }
   }
   for (int i = 0; i < n && best.warps; ++i) {
