@@ -67,16 +67,14 @@ int launch_cloud_gen_noalloc(int nd_layer, int cloud_top, int n_layer, int nd_pr
 static std::atomic<long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
-cudaError_t allow_shared(const void *kern, size_t bytes) {
-  cudaFuncAttributes fa{};
-  cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+cudaError_t allow_shared(const void *kern, size_t bytes, size_t fixed) {
+  if (bytes + fixed <= 48 * 1024) return cudaSuccess;   // the default limit, which covers both parts
   int dev = 0, most = 0;
-  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e == cudaSuccess && bytes + fa.sharedSizeBytes > (size_t)most) return cudaErrorInvalidValue;
-  // the default limit of 48 KB covers both parts
-  if (e == cudaSuccess && bytes + fa.sharedSizeBytes > 48 * 1024)
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes);
+  if (e == cudaSuccess && bytes + fixed > (size_t)most) return cudaErrorInvalidValue;
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fixed);
   if (e != cudaSuccess) cudaGetLastError();
   return e;
 }

@@ -212,7 +212,7 @@ int launch_prsc(const FluxParams &p, double *out, cudaStream_t st, char *msg, si
     snprintf(msg, len, "prescribed aerosol levels need %zu bytes of shared memory (limit %d)", smem, max_smem);
     return SOCGPU_I_ERR_RANGE;
   }
-  if (smem > 48 * 1024 && allow_shared((const void *)prsc_kernel, smem) != cudaSuccess) {
+  if (allow_shared((const void *)prsc_kernel, smem, 0) != cudaSuccess) {
     snprintf(msg, len, "shared memory request of %zu bytes refused", smem);
     return SOCGPU_I_ERR_RANGE;
   }

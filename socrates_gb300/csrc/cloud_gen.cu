@@ -344,10 +344,8 @@ static cudaError_t launch_generator(const GenArgs &a, cudaStream_t st) {
   const size_t bytes = gen_shared_bytes(std::max(ncl, 1), a.n_subcol);
   if (a.rng == SOCGPU_RNG_PHILOX && a.ipph == 0 &&
       (a.ioverlap == SOCGPU_IP_RAND || a.ioverlap == SOCGPU_IP_EXPONENTIAL_RAND) && bytes <= 100 * 1024) {
-    if (bytes > 48 * 1024) {
-      const cudaError_t e = allow_shared((const void *)cloud_gen_philox_kernel, bytes);
-      if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_shared((const void *)cloud_gen_philox_kernel, bytes, 0);
+    if (e != cudaSuccess) return e;
     cloud_gen_philox_kernel<<<(ncol + 31) / 32, 32 * std::min(16, a.n_subcol), bytes, st>>>(a, std::max(ncl, 1));
   } else {
     const int bs = gen_block(ncol);

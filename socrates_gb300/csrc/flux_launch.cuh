@@ -86,17 +86,15 @@ int launch_tau(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   }
   const size_t bytes = tau_bytes(q);
   auto kern = tau_single<NOSCAT, MCICA, SRC, S>(mb);
-  if (bytes > 48 * 1024) {
-    cudaError_t e = allow_shared((const void *)kern, bytes);
-    if (e != cudaSuccess) {
-      snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
-      return SOCGPU_I_ERR_RANGE;
-    }
+  cudaError_t e = allow_shared((const void *)kern, bytes, 0);
+  if (e != cudaSuccess) {
+    snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
+    return SOCGPU_I_ERR_RANGE;
   }
   if (p.n_profile <= 0) return 0;
   kern<<<(p.n_profile + q.tau.cols - 1) / q.tau.cols, warps * 32, bytes, st>>>(q);
   count_launch();
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) {
     snprintf(msg, len, "flux kernel launch failed: %s", cudaGetErrorString(e));
     return SOCGPU_I_ABORT_CALCULATION;
@@ -152,7 +150,7 @@ int prepare_tau(BatchGroup &g, char *msg, size_t len) {
   g.total = g.col_start[g.n_items];
   if (!shape.warps && warps == 8 && 2 * alone > g.total && tau_narrow(g.total, chip))
     kern = tau_batched<NOSCAT, MCICA, SRC, S>(3);
-  cudaError_t e = allow_shared((const void *)kern, bytes);
+  cudaError_t e = allow_shared((const void *)kern, bytes, (size_t)fixed);
   if (e != cudaSuccess) {
     snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
     return SOCGPU_I_ERR_RANGE;
@@ -206,12 +204,10 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   FluxParams q = p;
   q.band_batch = batch;
   auto kern = flux_kernel<R, MIX, S::P, S::CH, NOSCAT, MCICA, SRC>;
-  if (lay.bytes > 48 * 1024) {
-    cudaError_t e = allow_shared((const void *)kern, lay.bytes);
-    if (e != cudaSuccess) {
-      snprintf(msg, len, "shared memory request of %zu bytes refused: %s", lay.bytes, cudaGetErrorString(e));
-      return SOCGPU_I_ERR_RANGE;
-    }
+  cudaError_t e = allow_shared((const void *)kern, lay.bytes, 0);
+  if (e != cudaSuccess) {
+    snprintf(msg, len, "shared memory request of %zu bytes refused: %s", lay.bytes, cudaGetErrorString(e));
+    return SOCGPU_I_ERR_RANGE;
   }
   if (p.n_profile <= 0) return 0;
   int grid = p.n_profile;
@@ -227,7 +223,7 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   }
   kern<<<grid, threads, lay.bytes, st>>>(q);
   count_launch();
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (MCICA && p.region) scratch_free(q.region_scr, st);
   if (e != cudaSuccess) {
     snprintf(msg, len, "flux kernel launch failed: %s", cudaGetErrorString(e));
@@ -295,7 +291,7 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
     p.band_batch = batch;
   }
   const size_t dyn = smem;
-  cudaError_t e = allow_shared((const void *)kern, dyn);
+  cudaError_t e = allow_shared((const void *)kern, dyn, fa.sharedSizeBytes);
   if (e != cudaSuccess) {
     snprintf(msg, len, "shared memory request of %zu bytes refused: %s", dyn, cudaGetErrorString(e));
     return SOCGPU_I_ERR_RANGE;

@@ -49,19 +49,17 @@ int launch_phased_lp(const FluxParams &p, const TileConfig &cfg, cudaStream_t st
   FluxParams q = p;
   q.band_batch = batch;
   auto kern = flux_kernel_phased<R, MIX, NOSCAT, SRC, LPM>;
-  if (bytes > 48 * 1024) {
-    cudaError_t e = allow_shared((const void *)kern, bytes);
-    if (e != cudaSuccess) {
-      snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
-      return SOCGPU_I_ERR_RANGE;
-    }
+  cudaError_t e = allow_shared((const void *)kern, bytes, 0);
+  if (e != cudaSuccess) {
+    snprintf(msg, len, "shared memory request of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
+    return SOCGPU_I_ERR_RANGE;
   }
   if (p.n_profile <= 0) return 0;
   // warp 0 runs the serial recurrences, the others the coefficients and sums
   const int warps = cfg.warps_per_cta > 0 ? std::max(2, std::min(cfg.warps_per_cta, 8)) : 8;
   kern<<<p.n_profile, warps * 32, bytes, st>>>(q, gb);
   count_launch();
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) {
     snprintf(msg, len, "phased flux kernel launch failed: %s", cudaGetErrorString(e));
     return SOCGPU_I_ABORT_CALCULATION;

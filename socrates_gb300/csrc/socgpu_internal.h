@@ -380,13 +380,14 @@ inline bool phased_supported(const FluxParams &p) {
 
 void count_launch();
 
-// Lets kernel `kern` be launched with `bytes` of dynamic shared memory; called
-// before every launch, graph node or occupancy query that asks for them.  The
-// function's limit is one value for all calls, shapes and host threads, what
-// the current device grants a CTA less the kernel's static part: a limit set
-// to each launch's own size would fall between another launch's setting and
-// its use.  cudaErrorInvalidValue where the device does not grant the bytes.
-cudaError_t allow_shared(const void *kern, size_t bytes);
+// Lets kernel `kern`, which has `fixed` bytes of static shared memory, be
+// launched with `bytes` of dynamic shared memory; called before every launch,
+// graph node or occupancy query that asks for them.  The function's limit is
+// one value for all calls, shapes and host threads, what the current device
+// grants a CTA less the static part: a limit set to each launch's own size
+// would fall between another launch's setting and its use.
+// cudaErrorInvalidValue where the device does not grant the bytes.
+cudaError_t allow_shared(const void *kern, size_t bytes, size_t fixed);
 
 // Stream-ordered scratch of cloud-region launches, from a pool of the library
 // on the current device that keeps up to kScratchKeep bytes between launches
