@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "host_internal.h"
+#include "region_rows.h"
 
 namespace socgpu {
 
@@ -94,7 +95,7 @@ static cudaMemPool_t scratch_pool() {
   props.location.id = dev;
   cudaMemPool_t pool = nullptr;
   if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-  unsigned long long keep = kScratchKeep;
+  unsigned long long keep = kRegionRows;
   cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   pools[dev] = pool;
   return pool;
@@ -1625,11 +1626,30 @@ int make_group(socgpu_batch_s &b, const std::vector<int> &idx, int precision, in
 // Copy groups' tables to one device buffer (device pointers returned per group).
 int upload_groups(std::vector<BatchGroup> &groups, char *&dbuf, std::vector<FluxParams *> &d_items,
                   std::vector<long long *> &d_start, char *msg, size_t msg_len) {
-  size_t bytes = 0;
-  for (const BatchGroup &g : groups)
-    bytes += align256(sizeof(FluxParams) * g.n_items) + align256(sizeof(long long) * (g.n_items + 1)) + align256(g.scratch);
   if (dbuf) { cudaFree(dbuf); dbuf = nullptr; }
-  CUDA_TRY(cudaMalloc(&dbuf, std::max<size_t>(bytes, 256)));
+  // where memory is short, the cloud regions' classes run with fewer CTAs
+  for (;;) {
+    size_t bytes = 0;
+    bool more = false;
+    for (const BatchGroup &g : groups) {
+      bytes += align256(sizeof(FluxParams) * g.n_items) + align256(sizeof(long long) * (g.n_items + 1)) + align256(g.scratch);
+      more = more || (g.scratch && g.grid > 1);
+    }
+    const cudaError_t e = cudaMalloc(&dbuf, std::max<size_t>(bytes, 256));
+    if (e == cudaSuccess) break;
+    dbuf = nullptr;
+    cudaGetLastError();
+    if (e != cudaErrorMemoryAllocation || !more) {
+      set_msg(msg, msg_len, "no device memory for the batch (%zu bytes): %s", bytes, cudaGetErrorString(e));
+      return SOCGPU_I_ABORT_CALCULATION;
+    }
+    for (BatchGroup &g : groups)
+      if (g.scratch && g.grid > 1) {
+        g.scratch /= g.grid;
+        g.grid = (g.grid + 1) / 2;
+        g.scratch *= g.grid;
+      }
+  }
   size_t off = 0;
   d_items.clear(); d_start.clear();
   for (const BatchGroup &g : groups) {

@@ -6,6 +6,7 @@
 #include <cstdio>
 #include "flux_kernel.cuh"
 #include "flux_tau_kernel.cuh"
+#include "region_rows.h"
 
 namespace socgpu {
 
@@ -212,11 +213,16 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   if (p.n_profile <= 0) return 0;
   int grid = p.n_profile;
   if (MCICA && p.region) {
-    grid = std::min(grid, region_ctas(kern, threads, lay.bytes));
     q.region_rt = region_rt(p);
     q.region_stride = region_cta_bytes<R>(q);
-    if (scratch_alloc(&q.region_scr, q.region_stride * grid, st) != cudaSuccess) {
+    long long ctas = region_grid(std::min(grid, region_ctas(kern, threads, lay.bytes)), q.region_stride);
+    const bool rows = take_rows(ctas, q.region_stride, [&](size_t bytes) {
+      if (scratch_alloc(&q.region_scr, bytes, st) == cudaSuccess) return true;
       cudaGetLastError();
+      return false;
+    });
+    grid = (int)ctas;
+    if (!rows) {
       snprintf(msg, len, "no device memory for the cloud regions' rows");
       return SOCGPU_I_ABORT_CALCULATION;
     }
@@ -309,13 +315,13 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
   g.grid = (int)std::min<long long>(g.total, (long long)per_sm * n_sm);
   if (region) {
     // the resident CTAs' rows, sized for the widest item
-    g.grid = (int)std::min<long long>(g.total, (long long)std::min(per_sm, kRegionCtasPerSm) * n_sm);
     size_t cta = 0;
     for (int i = 0; i < g.n_items; ++i) {
       g.items[i].region_rt = region_rt(g.items[i]);
       cta = std::max(cta, region_cta_bytes<R>(g.items[i]));
     }
     for (int i = 0; i < g.n_items; ++i) g.items[i].region_stride = cta;
+    g.grid = (int)region_grid(std::min<long long>(g.total, (long long)std::min(per_sm, kRegionCtasPerSm) * n_sm), cta);
     g.scratch = cta * g.grid;
   }
   }

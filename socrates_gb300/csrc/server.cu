@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "host_internal.h"
+#include "region_rows.h"
 
 using namespace socgpu;
 using Clock = std::chrono::steady_clock;
@@ -292,8 +293,14 @@ void launch_wave(socgpu_server_s &S, StreamSlot &sl) {
     if (!g.scratch) g.grid = (int)std::min<long long>(g.total, 0x7fffffffLL);
     if (g.scratch) {
       void *rows = nullptr;
-      if (scratch_alloc(&rows, g.scratch, st) != cudaSuccess) {
+      long long ctas = g.grid;
+      const bool got = take_rows(ctas, g.scratch / g.grid, [&](size_t bytes) {
+        if (scratch_alloc(&rows, bytes, st) == cudaSuccess) return true;
         cudaGetLastError();
+        return false;
+      });
+      g.grid = (int)ctas;
+      if (!got) {
         for (void *q : scratch) scratch_free(q, st);
         fail_all(wave, SOCGPU_I_ABORT_CALCULATION, "no device memory for the cloud regions' rows");
         record_all(sl);

@@ -390,9 +390,9 @@ void count_launch();
 cudaError_t allow_shared(const void *kern, size_t bytes, size_t fixed);
 
 // Stream-ordered scratch of cloud-region launches, from a pool of the library
-// on the current device that keeps up to kScratchKeep bytes between launches
-// (socgpu_spectrum_release gives them back).
-constexpr size_t kScratchKeep = (size_t)512 << 20;
+// on the current device that keeps what one launch may take (kRegionRows)
+// between launches, so that a call after a synchronisation does not map it
+// again (socgpu_spectrum_release gives it back).
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st);
 void scratch_free(void *p, cudaStream_t st);
 void scratch_trim();
