@@ -219,8 +219,9 @@ __host__ __device__ inline SmemLayout make_layout(const FluxParams &p, int LP, i
   s.off_asym = take((size_t)nb * LP);
   s.off_fwd = take((size_t)nb * LP);
   s.off_amt = take((size_t)nb * max_abs * LP);
-  // FP64, solar: ksi_0 of each cell (a division saved per g-point)
-  s.off_ksi = (sizeof(R) == 8 && !lw) ? take((size_t)nb * LP) : o;
+  // FP64, solar: ksi_0 of each clear cell (a division saved per g-point; the
+  // cells of cloud regions form it themselves)
+  s.off_ksi = (sizeof(R) == 8 && !lw && !(mcica && p.region)) ? take((size_t)nb * LP) : o;
   s.off_bscal = take((size_t)nb * kBandScal);
   s.off_planck = lw ? take((size_t)nb * (LP + 1)) : o;
   s.off_dB = lw ? take((size_t)nb * LP) : o;
@@ -747,7 +748,7 @@ struct FluxKernel {
       __syncthreads();
       stage_boundary(p, S, col, bstart, nb, lw);
       if constexpr (kFP64 && !lw)
-        for (int q = threadIdx.x; q < nb * LP; q += nthreads)
+        for (int q = threadIdx.x; q < nb * LP && !(MCICA && p.region); q += nthreads)
           if (layer_of_slot(q % LP) < L) S.ksi[q] = ksi0_ref(p.i_2stream, S.asym[q], sec0);
       __syncthreads();
       if (S.raw) {
