@@ -15,7 +15,7 @@
 // the layer of trans_source_coeff.F90:144-200 is
 //
 //   T = 4 x e / W          R = h (S - D) / W
-//   1 - T     = (2 x (1-e)^2 + h (S + D)) / W
+//   1 - T     = (2 x (1-e)^2 + h (S + D)) / W      (T of thin solar layers from this)
 //   1 - T - R = (2 x (1-e)^2 + 2 h D) / W
 //
 // (gamma = (S - x)/(S + x) multiplied out, x^2 = S D), one division and no
@@ -124,6 +124,13 @@ __device__ __forceinline__ CellT cell_tau(const SchemeT &sc, int quad, float a, 
   const LayerT l = layer_tau(S, D, x, c.T);
   c.R = l.R; c.om = l.om;
   if constexpr (SRC == SOCGPU_IP_SOLAR) {
+    // the transmission of a thin layer from 1 - T: one rounding at 1 in place
+    // of four or five, which a column's layers multiply (GA9 short wave,
+    // upward flux against 64 bits: 1.1 times the error of the form of
+    // trans_source_coeff.F90 without this, 0.75 times with it, for 0.1 to 0.4 %
+    // of the time, 3 % at 1000 x 60.  In the infra-red, where the sources
+    // dominate, it changes nothing)
+    if (l.omt < 0.5f) c.T = 1.0f - l.omt;
     const float z = tau * sec0;
     c.T0 = exp2f(-kLog2e * z);
     const float omt0 = one_minus_exp(z, c.T0);
