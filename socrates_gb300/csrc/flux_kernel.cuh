@@ -444,7 +444,7 @@ struct FluxKernel {
     Acc *acc;
     // the mixed kernels' depths and accumulators (flux_tau_kernel.cuh)
     float4 *opt, *copt;
-    float *tkd, *pl, *accd;
+    float *tkd, *pl, *accd, *anc;
     float2 *acc2;
     // the column's raw inputs (null: read them from global memory)
     const double *raw;

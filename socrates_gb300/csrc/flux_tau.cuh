@@ -32,9 +32,9 @@
 //
 // so the chunk is eliminated once (solver_homogen_direct.F90:94-131, from
 // the top down).  A prefix scan of the composites and a suffix scan of the
-// chunks' affine maps close the column.  The downward fluxes are not
-// accumulated per g-point: the net flux is the top's less the divergences
-// above, summed with a compensated scan once per column.
+// chunks' affine maps close the column.  The downward fluxes are accumulated
+// per g-point at the chunk tops and at the surface only: between, they follow
+// once per column from the divergences (TauKernel::finish).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -175,15 +175,6 @@ __device__ __forceinline__ CompT stack_tau(const CompT &a, const CompT &b) {   /
   return o;
 }
 
-// Sum of two-word values (hi, lo), the rounding of the leading sum kept.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  const float s = __fadd_rn(a.x, b.x), t = __fadd_rn(s, -a.x);
-  const float err = __fadd_rn(__fadd_rn(a.x, -__fadd_rn(s, -t)), __fadd_rn(b.x, -t));
-  const float lo = __fadd_rn(err, __fadd_rn(a.y, b.y));
-  const float hi = __fadd_rn(s, lo);
-  return make_float2(hi, __fadd_rn(lo, -__fadd_rn(hi, -s)));
-}
-
 // ---------------------------------------------------------------------------
 // The solve of one monochromatic column.  Sm is FluxKernel's view of the
 // shared memory; slots as there (lane r's j-th layer in slot j P + r).
@@ -315,12 +306,14 @@ struct TauSolve {
     return f_inc * bottom;
   }
 
-  // acc2: the group's (up, divergence) per slot, slot LP holding (up at the
-  // top, down at the top); accd: its direct flux per slot (solar) or its
-  // downward flux (without scattering).  w: the weight.
+  // acc2: the group's (up, divergence) per slot, slot LP holding the upward
+  // flux at the top; accd: its direct flux per slot (solar) or its downward
+  // flux (without scattering); anc: the downward flux at the top of each
+  // lane's chunk and (entry P) at the surface (with scattering).  w: the weight.
   // buf: the lane's kBlock cells (McICA), 32 lanes apart.
   __device__ static __forceinline__ void solve(const FluxParams &p, const Sm &S, const Band &b, int r, float sec0,
-                                               const float *bs, float w, float2 *acc2, float *accd, float4 *buf) {
+                                               const float *bs, float w, float2 *acc2, float *accd, float *anc,
+                                               float4 *buf) {
     const SchemeT sc(p);
     const float f_inc_down = bs[0], alb = bs[2];
     float fd = 0.0f, src = 0.0f;
@@ -335,7 +328,7 @@ struct TauSolve {
       fd = bs[1] * beam_scan(t, r, bottom);
       if (b.tkd) bottom = unscaled_beam(p, S, b, r, sec0, bs[1], w, accd);
       else {
-        if (r == 0) accd[LP] += w * fd;
+        if (r == 0) accd[LP] = fmaf(w, fd, accd[LP]);
         bottom *= bs[1];
       }
       src = (bs[3] - alb) * bottom;
@@ -465,7 +458,7 @@ struct TauSolve {
       if (b.tkd) {
         bottom = unscaled_beam(p, S, b, r, sec0, bs[1], w, accd);
       } else {
-        if (r == 0) accd[LP] += w * fd;
+        if (r == 0) accd[LP] = fmaf(w, fd, accd[LP]);
 #pragma unroll
         for (int j = 0; j < CH; ++j) accd[j * P + r] += (w * fd) * bt[j];
       }
@@ -495,6 +488,7 @@ struct TauSolve {
       // the surface closes the last chunk: F_up = alb F_dn + src
       const float rb = fmaf(c.T * rho, A0, c.R2), sb = fmaf(c.T, fmaf(rho, B0, sig), c.Sd);
       f_surf = fmaf(alb, sb, src) / fmaf(-alb, rb, 1.0f);
+      anc[P] = fmaf(w, fmaf(rb, f_surf, sb), anc[P]);
       B = fmaf(A, f_surf, B); A = 0.0f;
     }
 #pragma unroll
@@ -505,6 +499,7 @@ struct TauSolve {
     float fu = __shfl_down_sync(0xffffffffu, B, 1, P);     // F_up at the chunk bottom
     if (r == P - 1) fu = f_surf;
     const float fdt = fmaf(rho, B, sig);                   // B: F_up at this chunk's top
+    anc[r] = fmaf(w, fdt, anc[r]);
 #pragma unroll
     for (int j = CH - 1; j >= 0; --j) {
       const int s = j * P + r;
@@ -515,7 +510,7 @@ struct TauSolve {
       acc2[s] = v;
       fu = fmaf(ca[j], fu, fmaf(ce[j], fdt, gj));
     }
-    if (r == 0) { acc2[LP].x += w * fu; acc2[LP].y += w * f_inc_down; }
+    if (r == 0) acc2[LP].x += w * fu;
   }
 };
 

@@ -164,7 +164,7 @@ struct TauLayout {
   int acc_stride, accd_stride;      // accumulators of a group: (up, divergence) pairs, direct fluxes
   unsigned stride;
   unsigned opt, copt, tkd, amt, aux, bscal, planck, dB, dB2, pl, p, t, mass, frac, csub, lkf, lki, sbf, sbj, scr;
-  unsigned acc2, accd;
+  unsigned acc2, accd, anc;
 };
 
 // Everything a flux kernel launch reads, as device pointers with the
