@@ -153,7 +153,7 @@ struct SmemLayout {
   size_t off_phf_nc, off_fwd_nc, off_c_ke, off_c_ks, off_c_ka, off_c_phf, off_c_fwd;
   size_t off_wcld, off_frac, off_csub;
   size_t off_aux, off_lkf, off_lki, off_sbf, off_sbj, off_kscr;
-  size_t off_ovl, off_nct, off_t0d, off_frr;
+  size_t off_ovl, off_nct, off_t0d, off_frr, off_rwt;
   size_t off_acc;
   // the column's FP64 inputs, fetched into shared memory ahead of staging
   // (offsets in doubles from off_acc, whose space they share); raw_on false
@@ -163,7 +163,7 @@ struct SmemLayout {
   size_t bytes;
 };
 
-// Rows of a group's scratch for the two-region solve (cloud regions): the
+// Rows of the two-region solve of a g-point (cloud regions): the
 // clear (free) and cloudy coefficients of each layer, the elimination
 // coefficients of the solver, the level fluxes and the layer divergence.
 enum RegRow {
@@ -176,7 +176,7 @@ enum RegRow {
   kRgVT = kRegRows, kRgVR, kRgVT0, kRgVC1, kRgVC2, kRgVOM, kRgVT0D, kRegRows3
 };
 // The solver's elimination coefficients, kept in FP64 in every build: the
-// serial solve runs on one lane in FP64 from the coefficients of the layers.
+// serial solve of a g-point runs on one thread in FP64 from the coefficients of the layers.
 enum RegDRow { kRgB11, kRgB21, kRgB22, kRgG11, kRgG12, kRgG21, kRgG22, kRgH1, kRgH2, kRegDRows,
                // three regions (Hogan's form): the convective region's
                // elimination coefficients and its solar sources in FP64
@@ -192,6 +192,7 @@ struct Strided {
   int st;
   __device__ __forceinline__ T &operator[](int i) const { return p[(size_t)i * st]; }
 };
+constexpr int kRegionRt = 64;         // most g-points that a CTA solves at a time (region_rt)
 template <class R>
 __host__ __device__ inline size_t region_cta_bytes(const FluxParams &p) {
   const size_t rows = p.triple ? kRegRows3 : kRegRows, rowsd = p.triple ? kRegDRows3 : kRegDRows;
@@ -248,11 +249,12 @@ __host__ __device__ inline SmemLayout make_layout(const FluxParams &p, int LP, i
   // per-group scratch row for k of per-term scaled absorbers
   s.off_kscr = p.term_scr ? take((size_t)n_groups * LP) : o;
   // cloud regions: the column's interface coefficients and cloud top (the
-  // solves' rows lie in global memory, RegionScratch)
+  // solves' rows lie in global memory, region_cta_bytes)
   const bool region = mcica && p.region;
   const bool triple = region && p.triple;
   s.off_ovl = region ? take((size_t)(triple ? 18 : 8) * (LP + 1)) : o;
   s.off_nct = region ? take_int(4) : o;
+  s.off_rwt = region ? take(kRegionRt) : o;   // the weights of the g-points that are solved together
   // three regions: the stratiform and convective shares of each layer's
   // cloud (frac_region), by layer
   s.off_frr = triple ? take((size_t)2 * LP) : o;
@@ -441,6 +443,7 @@ struct FluxKernel {
     int *lki, *sbj;
     R *ovl, *t0d, *frr;
     int *nct;
+    R *rwt;
     Acc *acc;
     // the mixed kernels' depths and accumulators (flux_tau_kernel.cuh)
     float4 *opt, *copt;
@@ -468,6 +471,7 @@ struct FluxKernel {
     s.sbf = (R *)(smem + l.off_sbf); s.sbj = (int *)(smem + l.off_sbj);
     s.scr = (R *)(smem + l.off_kscr) + (size_t)(threadIdx.x / P) * LP;
     s.ovl = (R *)(smem + l.off_ovl); s.nct = (int *)(smem + l.off_nct);
+    s.rwt = (R *)(smem + l.off_rwt);
     s.t0d = (R *)(smem + l.off_t0d);
     s.frr = (R *)(smem + l.off_frr);
     s.acc = (Acc *)(smem + l.off_acc);
@@ -1869,6 +1873,11 @@ struct FluxKernel {
     const int t0 = ((int)threadIdx.x + nt - (int)(blockIdx.x * 64u) % nt) % nt;
     for (int g0 = g_lo; g0 < g_hi; g0 += st) {
       const int ng = min(st, g_hi - g0);
+      for (int t = threadIdx.x; t < ng; t += nt) {
+        const GPoint &gp = p.gpoints[g0 + t];
+        const R wb = S.bscal[(gp.band - bstart) * kBandScal + 5];
+        S.rwt[t] = kFP64 ? (R)(wb * gp.weight) : (R)(wb * gp.weight_f);
+      }
       for (int q = threadIdx.x; q < L * st; q += nt) {
         const int i = q / st, t = q - i * st;
         if (t < ng) region_cell(p, S, X + t, st, g0 + t, bstart, i, nct, sec0);
@@ -1880,19 +1889,20 @@ struct FluxKernel {
         else region_serial(p, S, X + t, Y + t, st, nct, L, lw, bs[0], bs[1], bs[2], bs[3], bs[4]);
       }
       __syncthreads();
-      // a thread sums one level of one flux over the g-points
+      // a thread sums one level of one flux over the g-points, in eight parts (the
+      // rounding of one running sum grows with all of them: 1.06 times the
+      // error of the groups' sums that the McICA kernels take, 0.98 in parts)
       for (int q = threadIdx.x; q < 4 * (L + 1); q += nt) {
         const int v = q / (L + 1), i = q - v * (L + 1);
         if ((v == 2 && lw) || (v == 3 && i == L)) continue;
         const int row = v == 0 ? kRgFU : v == 1 ? kRgFD : v == 2 ? kRgFDIR : kRgDIV;
         const R *x = X + ((size_t)row * (L + 1) + i) * st;
-        R sum = R(0);
-        for (int t = 0; t < ng; ++t) {
-          const GPoint &gp = p.gpoints[g0 + t];
-          const R *bs = S.bscal + (gp.band - bstart) * kBandScal;
-          const R w = kFP64 ? (R)(bs[5] * gp.weight) : (R)(bs[5] * gp.weight_f);
-          sum += w * x[t];
-        }
+        R part[8] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
+        for (int t = 0; t < ng; t += 8)
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (t + k < ng) part[k] += S.rwt[t + k] * x[t + k];
+        const R sum = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
         // the divergence of layer i sits at its bottom level's slot
         S.acc[(size_t)v * (LP + 1) + (v == 3 ? slot(i) : level_slot(i))] += sum;
       }
@@ -1900,9 +1910,9 @@ struct FluxKernel {
     }
   }
 
-  // The serial part of the two-region solve, on one lane, in FP64 in every
-  // build (the FP32 coefficients of the layers are its inputs): rows as
-  // solve_region leaves them; writes the level fluxes (diffuse in the
+  // The serial part of the two-region solve of a g-point, on one thread, in FP64
+  // in every build (the FP32 coefficients of the layers are its inputs): rows as
+  // region_cell leaves them; writes the level fluxes (diffuse in the
   // solar), the direct flux and the layer divergence.  Layers i are 0-based
   // here; interface i lies below layer i-1 (0: the top).
   __device__ static __noinline__ void region_serial(const FluxParams &p, const Smem &S, R *X, double *Y, int st, int nct,
@@ -2088,9 +2098,9 @@ struct FluxKernel {
   }
 
   // The serial part of the three-region solve (clear, stratiform and
-  // convective) on one lane, in FP64 in every build: triple_solar_source.F90:
+  // convective) of a g-point, on one thread, in FP64 in every build: triple_solar_source.F90:
   // 160-400, the ground sources of triple_column.F90:380-410 and
-  // solver_triple_hogan.F90:200-410.  Rows as solve_region leaves them, the
+  // solver_triple_hogan.F90:200-410.  Rows as region_cell leaves them, the
   // interface coefficients of stage_regions3 (v_jk row 3 j + k, u_jk row
   // 9 + 3 j + k); writes the level fluxes (diffuse in the solar), the direct
   // flux and the layer divergence.  Layers i are 0-based here; interface i

@@ -48,7 +48,7 @@ auto tau_batched(int mb) {
 
 // Threads that solve a cloud-region column's g-points at a time: whole warps
 // for the calls of up to 64 g-points.
-inline int region_rt(const FluxParams &p) { return std::min(64, (p.g_end - p.g_begin + 15) / 16 * 16); }
+inline int region_rt(const FluxParams &p) { return std::min(kRegionRt, (p.g_end - p.g_begin + 15) / 16 * 16); }
 
 // Resident CTAs of a cloud-region launch: four of four warps to an SM (solar,
 // 1025 x 70 x 48: 904 us; two of eight warps 1232, four of two 987).

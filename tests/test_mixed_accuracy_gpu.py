@@ -66,3 +66,19 @@ def test_downward_flux_under_thick_cloud(gpu_lib, solar, L, mmr, bound):
         assert got.min() >= 0.0
     else:
         assert np.abs(got - ref).max() <= 4 * L * 2.0 ** -24 * ref.max()
+
+
+@pytest.mark.parametrize("L,down,direct", [(38, 1.24e-7, 1.87e-7), (70, 1.68e-7, 2.77e-7), (137, 2.78e-7, 4.49e-7)])
+def test_sums_over_g_points_of_cloud_regions(gpu_lib, L, down, direct):
+    """Relative root-mean-square errors of 64 two-region solar columns: the
+    regions are solved in FP64, so what the sums over the g-points round shows."""
+    sp = synth.sw_spectrum(2, 8, clouds=True)
+    col = synth.atmosphere(64, L, sp.type_absorb, 1)
+    synth.add_sw_surface(col, sp.n_band, 1)
+    synth.add_clouds(col, 1, 16)
+    ctl = R.sw_control(i_cloud=abi.IP_CLOUD_MIX_MAX, i_solver=abi.IP_SOLVER_MIX_DIRECT_HOGAN)
+    ref = R.radiance_calc(ctl, sp, col)
+    got = R.radiance_calc(replace(ctl, precision=abi.PRECISION_MIXED), sp, col)
+    for k, bound in (("flux_down", down), ("flux_direct", direct)):
+        err = np.sqrt(((got[k] - ref[k]) ** 2).mean() / (ref[k] ** 2).mean())
+        assert err <= bound, (k, err)
