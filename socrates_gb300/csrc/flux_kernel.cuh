@@ -159,6 +159,7 @@ struct SmemLayout {
   // (offsets in doubles from off_acc, whose space they share); raw_on false
   // leaves staging on direct global loads
   int raw_on, raw_n;
+  int ksi_on;
   int r_p, r_t, r_mass, r_gas, r_mmr, r_mabs, r_msca, r_masy, r_sol, r_zen, r_alb, r_tg, r_fg, r_tl;
   size_t bytes;
 };
@@ -220,9 +221,10 @@ __host__ __device__ inline SmemLayout make_layout(const FluxParams &p, int LP, i
   s.off_asym = take((size_t)nb * LP);
   s.off_fwd = take((size_t)nb * LP);
   s.off_amt = take((size_t)nb * max_abs * LP);
-  // FP64, solar: ksi_0 of each clear cell (a division saved per g-point; the
-  // cells of cloud regions form it themselves)
-  s.off_ksi = (sizeof(R) == 8 && !lw && !(mcica && p.region)) ? take((size_t)nb * LP) : o;
+  // FP64, solar: ksi_0 of each clear cell (a division saved per g-point),
+  // unless its row does not fit; the cells of cloud regions form it themselves
+  s.ksi_on = sizeof(R) == 8 && !lw && !(mcica && p.region) && !p.no_ksi;
+  s.off_ksi = s.ksi_on ? take((size_t)nb * LP) : o;
   s.off_bscal = take((size_t)nb * kBandScal);
   s.off_planck = lw ? take((size_t)nb * (LP + 1)) : o;
   s.off_dB = lw ? take((size_t)nb * LP) : o;
@@ -459,7 +461,7 @@ struct FluxKernel {
     s.p = (R *)(smem + l.off_p); s.t = (R *)(smem + l.off_t); s.mass = (R *)(smem + l.off_mass);
     s.kgt = (R *)(smem + l.off_kgt); s.kes = (R *)(smem + l.off_kes); s.kabs = (R *)(smem + l.off_kabs);
     s.asym = (R *)(smem + l.off_asym); s.fwd = (R *)(smem + l.off_fwd); s.amt = (R *)(smem + l.off_amt);
-    s.ksi = (R *)(smem + l.off_ksi);
+    s.ksi = l.ksi_on ? (R *)(smem + l.off_ksi) : nullptr;
     s.bscal = (R *)(smem + l.off_bscal);
     s.planck = (R *)(smem + l.off_planck); s.dB = (R *)(smem + l.off_dB); s.dB2 = (R *)(smem + l.off_dB2);
     s.phf_nc = (R *)(smem + l.off_phf_nc); s.fwd_nc = (R *)(smem + l.off_fwd_nc);
@@ -752,7 +754,7 @@ struct FluxKernel {
       __syncthreads();
       stage_boundary(p, S, col, bstart, nb, lw);
       if constexpr (kFP64 && !lw)
-        for (int q = threadIdx.x; q < nb * LP && !(MCICA && p.region); q += nthreads)
+        for (int q = threadIdx.x; S.ksi && q < nb * LP; q += nthreads)
           if (layer_of_slot(q % LP) < L) S.ksi[q] = ksi0_ref(p.i_2stream, S.asym[q], sec0);
       __syncthreads();
       if (S.raw) {
@@ -1590,7 +1592,7 @@ struct FluxKernel {
         const int i = r * CH + j, s = j * P + r;
         if (i < L) {
           cell_coef(p, kgt_b[s], kes_b[s], kabs_b[s], kgv[j], S.mass[s], asym_b[s], fwd_b[s], sec0,
-                    T[j], Rf[j], T0[j], c1[j], c2[j], om[j], S.ksi + (size_t)bi * LP + s);
+                    T[j], Rf[j], T0[j], c1[j], c2[j], om[j], S.ksi ? S.ksi + (size_t)bi * LP + s : nullptr);
         } else {
           T[j] = R(1); Rf[j] = R(0); T0[j] = R(1); c1[j] = R(0); c2[j] = R(0); om[j] = R(0);
         }
@@ -2316,7 +2318,7 @@ struct FluxKernel {
           }
           if (!cloudy) {
             cell_coef(p, kgt_b[s], kes_b[s], kabs_b[s], kg, S.mass[s], asym_b[s], fwd_b[s], sec0,
-                      T[jj], Rf[jj], T0[jj], c1[jj], c2[jj], om[jj], S.ksi + (size_t)bi * LP + s);
+                      T[jj], Rf[jj], T0[jj], c1[jj], c2[jj], om[jj], S.ksi ? S.ksi + (size_t)bi * LP + s : nullptr);
             if (t0d) t0d[s] = t0_unscaled(kgt_b[s], kg, S.mass[s], sec0);
           } else {
             // mcica_sample.F90:472-700 then mcica_column.F90:336-470: each

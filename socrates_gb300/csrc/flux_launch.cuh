@@ -191,18 +191,19 @@ int try_launch(const FluxParams &p, const TileConfig &cfg, cudaStream_t st, char
   const int given = cfg.warps_per_cta > 0 ? cfg.warps_per_cta : 8;
   int warps = MCICA && p.region ? std::min(given, kRegionWarps) : given, batch = nb;
   SmemLayout lay{};
+  FluxParams q = p;
   for (;;) {
-    lay = make_layout<R>(p, S::P * S::CH, S::P, batch, warps * 32 / S::P, MCICA,
+    lay = make_layout<R>(q, S::P * S::CH, S::P, batch, warps * 32 / S::P, MCICA,
                          FluxKernel<R, MIX, S::P, S::CH, NOSCAT, MCICA, SRC>::kRawFetch);
     if ((long long)lay.bytes <= max_smem) break;
     if (batch > 1) { --batch; continue; }
     if (warps > 1) { warps /= 2; batch = nb; continue; }
+    if (lay.ksi_on) { q.no_ksi = 1; batch = nb; continue; }
     snprintf(msg, len, "one band of %d layers needs %zu bytes of shared memory (limit %d)", p.n_layer, lay.bytes,
              max_smem);
     return SOCGPU_I_ERR_RANGE;
   }
   const int threads = warps * 32;
-  FluxParams q = p;
   q.band_batch = batch;
   auto kern = flux_kernel<R, MIX, S::P, S::CH, NOSCAT, MCICA, SRC>;
   cudaError_t e = allow_shared((const void *)kern, lay.bytes, 0);
@@ -257,10 +258,9 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
   const bool region = MCICA && g.n_items > 0 && g.items[0].region;
   const int given = g.tile.warps_per_cta > 0 ? g.tile.warps_per_cta : 8;
-  const int warps = region ? std::min(given, kRegionWarps) : given;
-  const int n_groups = warps * 32 / S::P;
+  int warps = region ? std::min(given, kRegionWarps) : given;
   auto bytes_of = [&](const FluxParams &p, int batch) {
-    return make_layout<R>(p, S::P * S::CH, S::P, batch, n_groups, MCICA,
+    return make_layout<R>(p, S::P * S::CH, S::P, batch, warps * 32 / S::P, MCICA,
                           FluxKernel<R, MIX, S::P, S::CH, NOSCAT, MCICA, SRC>::kRawFetch).bytes;
   };
   auto kern = flux_kernel_batched<R, MIX, S::P, S::CH, NOSCAT, MCICA, SRC>;
@@ -278,11 +278,21 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
   // in batches
   size_t smem = 0;
   for (int i = 0; i < g.n_items; ++i) {
-    const FluxParams &p = g.items[i];
+    FluxParams &p = g.items[i];
     if (p.n_layer > S::P * S::CH) {
       snprintf(msg, len, "batch %d has %d layers, more than the %d of its tile", i, p.n_layer, S::P * S::CH);
       return SOCGPU_I_ERR_RANGE;
     }
+    // fewer warps for all, then no ksi_0 row, where one band does not fit
+    while (bytes_of(p, 1) > dyn_cap && warps > 1) warps /= 2;
+    p.no_ksi = bytes_of(p, 1) > dyn_cap;
+    if (bytes_of(p, 1) > dyn_cap) {
+      snprintf(msg, len, "batch %d: one band needs %zu bytes of shared memory (limit %zu)", i, bytes_of(p, 1), dyn_cap);
+      return SOCGPU_I_ERR_RANGE;
+    }
+  }
+  for (int i = 0; i < g.n_items; ++i) {
+    const FluxParams &p = g.items[i];
     smem = std::max(smem, bytes_of(p, p.last_band - p.first_band + 1));
   }
   smem = std::min(smem, dyn_cap);
@@ -290,10 +300,6 @@ int try_prepare(BatchGroup &g, char *msg, size_t len, bool &done) {
     FluxParams &p = g.items[i];
     int batch = p.last_band - p.first_band + 1;
     while (batch > 1 && bytes_of(p, batch) > smem) --batch;
-    if (bytes_of(p, batch) > smem) {
-      snprintf(msg, len, "batch %d: one band needs %zu bytes of shared memory (limit %zu)", i, bytes_of(p, 1), smem);
-      return SOCGPU_I_ERR_RANGE;
-    }
     p.band_batch = batch;
   }
   const size_t dyn = smem;

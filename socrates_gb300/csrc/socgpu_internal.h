@@ -184,6 +184,7 @@ struct FluxParams {
   int width;                        // columns of the caller's call, of which n_profile may be a window
   int g_begin, g_end;               // g-point range of the band range
   int max_abs;                      // most absorbers of any band in the range (>= 1)
+  int no_ksi;                       // ksi_0 formed per cell, its staged row left out (set by the launcher)
   int band_batch;                   // bands staged in shared memory at a time (set by the launcher)
   // spectrum
   const BandInfo *bands;
