@@ -12,6 +12,8 @@ demangled -k regex:<kernel> -s 1 -c 1 python -m socrates_gb300.profile_cases
                     shortwave configuration (flux_kernel<double ...>)
   lwns              mixed infra-red no-scattering kernel, 30000 x 60
   mcica_sw          mixed solar McICA kernel, 8192 x 85, 16 subcolumns
+  region            mixed solar two-region kernel, 2048 x 70
+  sw                mixed solar kernel, 10000 columns x 100 layers
   batched           the multi-batch kernel over 256 mixed requests
   cloud_gen         the McICA subcolumn generator, 8192 x 85
   prsc              prescribed aerosol properties and the solar kernel after
@@ -27,7 +29,7 @@ from . import abi, synth
 from . import radiance as R
 from .device import DeviceCase
 
-CASES = ("fp64_sw", "lwns", "mcica_sw", "batched", "cloud_gen", "prsc", "phased", "fp64_lwns_phased")
+CASES = ("fp64_sw", "lwns", "mcica_sw", "region", "sw", "batched", "cloud_gen", "prsc", "phased", "fp64_lwns_phased")
 
 
 def run(mode: str) -> None:
@@ -46,6 +48,17 @@ def run(mode: str) -> None:
         c_sub, nsc = R.cloud_gen(col, 16, abi.IP_EXPONENTIAL_RAND, abi.RNG_PHILOX)
         mc = R.set_cld_mcica(sw, col, abi.IP_SOLAR, abi.IP_MCICA_SINGLE_SAMPLING, c_sub=c_sub, n_subcol_cld=nsc)
         case = DeviceCase(R.sw_control(i_cloud=abi.IP_CLOUD_MCICA, precision=abi.PRECISION_MIXED), sw, col, mc)
+    elif mode == "region":
+        sp = synth.sw_spectrum(2, 8, clouds=True)
+        col = synth.atmosphere(2048, 70, sp.type_absorb, 2)
+        synth.add_sw_surface(col, sp.n_band, 2)
+        synth.add_clouds(col, 2, 16)
+        no_subcol = R.McicaState(1, 1, None, None, None, None, None, None)
+        case = DeviceCase(R.sw_control(i_cloud=abi.IP_CLOUD_MIX_MAX, i_solver=abi.IP_SOLVER_MIX_DIRECT_HOGAN,
+                                       precision=abi.PRECISION_MIXED), sp, col, no_subcol)
+    elif mode == "sw":
+        sp, col = synth.config2(10000, 100, 2)
+        case = DeviceCase(R.sw_control(l_aerosol_mode=True, precision=abi.PRECISION_MIXED), sp, col)
     elif mode == "batched":
         from .batch import Batch
         from .workload import Pools, request_specs
